@@ -445,7 +445,11 @@ mgc_status mgc_autotune_rewind(mgc_sim* sim, int64_t steps_per_trial, mgc_tune_r
  * steps (mgc_set_window) are delivered before it, then every neuron advances
  * the W steps with its state in registers, two grid barriers per window.
  * Default: 2 when the minimum delay is >= 4, else 1; the autotuner may pick
- * another.  If the device cannot keep all blocks of a group resident, the
+ * another.  By default, and when the autotuner finds it fastest, a network
+ * whose state fits on the chip runs the tiled step group in the place of that
+ * mode (one block per SM keeps its neurons' state and inputs in shared memory
+ * and delivers every spike to its own targets from a copy of the synapses cut
+ * by block); a mode set here runs as described.  If the device cannot keep all blocks of a group resident, the
  * call falls back to 0.  Results are the same in every mode; while a schedule mode other than
  * static, recording or calibration is on, graphs are used.  All waits are
  * bounded (a time-out makes mgc_sync return MGC_ERR_CUDA).  No reference

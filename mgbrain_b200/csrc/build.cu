@@ -479,6 +479,7 @@ mgc_status finish_build(mgc_sim* s)
     }
     a.M = s->M;
     CKS(launch_shapes(s));
+    CKS(build_tiles(s));
     CK(cudaStreamSynchronize(s->stream));
     return MGC_OK;
 }
@@ -634,10 +635,8 @@ namespace mgc {
 mgc_status launch_shapes(mgc_sim* s)
 {
     StepArgs& a = s->a;
-    cudaDeviceProp prop;
-    CK(cudaGetDeviceProperties(&prop, s->device));
-    const int sms = prop.multiProcessorCount;
-    int occ = 0;
+    int sms = 0, occ = 0;
+    CKS(device_attr(cudaDevAttrMultiProcessorCount, s->device, &sms));
     if (a.deferred) {
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, deliver_kernel(s), kPushBlock, 0));
         s->deliver_grid = sms * std::max(1, occ);
@@ -722,6 +721,8 @@ mgc_status build_set_fx(mgc_sim* s, bool hetero, int32_t fx_shift)
 }
 
 mgc_status build_finish(mgc_sim* s) { return finish_build(s); }
+
+mgc_status scan_offsets(uint32_t* v, int64_t count, cudaStream_t st) { return exclusive_scan(v, count, st); }
 
 // The CSR (and the method's extra layouts) of a network handed over as a
 // device-resident synapse list in synapse-list order: sources, targets,
@@ -1237,6 +1238,7 @@ extern "C" mgc_status mgc_set_accumulation(mgc_sim* s, int32_t mode)
     }
     a.fx = fx;
     CKS(launch_shapes(s));
+    CKS(build_tiles(s));
     CK(cudaStreamSynchronize(s->stream));
     return MGC_OK;
 }

@@ -49,11 +49,18 @@ mgc_status pick_device(int device)
     }
     if (device < 0 || device >= count) return fail(MGC_ERR_INVALID, "device %d out of range", device);
     CK(cudaSetDevice(device));
-    cudaDeviceProp prop;
-    CK(cudaGetDeviceProperties(&prop, device));
-    if (prop.major != 10)
-        return fail(MGC_ERR_NODEVICE, "device %d is sm_%d%d; this library holds sm_100a code only", device,
-                    prop.major, prop.minor);
+    int major = 0, minor = 0;
+    CKS(device_attr(cudaDevAttrComputeCapabilityMajor, device, &major));
+    CKS(device_attr(cudaDevAttrComputeCapabilityMinor, device, &minor));
+    if (major != 10)
+        return fail(MGC_ERR_NODEVICE, "device %d is sm_%d%d; this library holds sm_100a code only", device, major,
+                    minor);
+    return MGC_OK;
+}
+
+mgc_status device_attr(cudaDeviceAttr attr, int device, int* value)
+{
+    CK(cudaDeviceGetAttribute(value, attr, device));
     return MGC_OK;
 }
 

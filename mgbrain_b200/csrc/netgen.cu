@@ -298,10 +298,10 @@ mgc_status gen_prob(mgc_sim* s, MGBrain::Mt19937& g, uint64_t max_num, uint64_t 
         if (gen_num) k_fill<<<grid_for((int64_t)gen_num), 256, 0, s->stream>>>((int64_t)gen_num, src, src0, tar, tar0);
         return MGC_OK;
     }
-    cudaDeviceProp prop;
-    CK(cudaGetDeviceProperties(&prop, s->device));
+    int sms = 0;
+    CKS(device_attr(cudaDevAttrMultiProcessorCount, s->device, &sms));
     const uint64_t want = (max_num + kStretchMin - 1) / kStretchMin;
-    const size_t B = (size_t)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)prop.multiProcessorCount));
+    const size_t B = (size_t)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)sms));
     const uint64_t C = (max_num + B - 1) / B;
     const std::vector<MGBrain::Mt19937> st = stretch_starts(g, B, C);
     std::vector<uint32_t> words(B * kMtN);

@@ -291,14 +291,25 @@ mgc_status mgc_run(mgc_sim* s, int64_t steps)
         // barrier between steps (or the pipelined arrive/wait) instead of a launch
         const int p = s->persistent, v = s->fused_variant;
         while (left > 0) {
-            int32_t n = (int32_t)std::min<int64_t>(left, kPersistentSteps);
+            int32_t n = (int32_t)std::min<int64_t>(left, s->tile_on ? kTileSteps : kPersistentSteps);
             // the schedule trace only while the scheduler's graph runs
             StepArgs ga = s->a;
             ga.trace = nullptr;
             void* args[] = {&ga, &n};
-            CK(cudaMemsetAsync(s->a.bar, 0, 4 * sizeof(unsigned int), s->stream));  // clean barriers
+            if (!s->tile_on)
+                CK(cudaMemsetAsync(s->a.bar, 0, 4 * sizeof(unsigned int), s->stream));  // clean barriers
             cudaError_t e;
-            if (p == 3) {
+            if (s->tile_on) {
+                void* targs[] = {&ga, &s->tile, &n};
+                e = cudaLaunchCooperativeKernel((const void*)tile_kernel(s), dim3(s->tile.T), dim3(kTileThreads),
+                                                targs, s->tile_smem, s->stream);
+                if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+                    cudaGetLastError();  // not all resident here: the other step groups
+                    s->tile_on = false;
+                    continue;
+                }
+                if (e == cudaSuccess) s->tile.epoch += (uint32_t)((n + s->tile.W - 1) / s->tile.W + 1);  // windows, the end
+            } else if (p == 3) {
                 int32_t w = s->window;
                 // a window of w steps holds w buffers; each instantiation
                 // is compiled for one cycle (3, or 7 above 4 steps)

@@ -15,6 +15,7 @@
 #include "../../include/mgc.h"
 #include "kernels.cuh"
 #include "sched_state.h"
+#include "tile.cuh"
 
 namespace mgc {
 
@@ -53,6 +54,7 @@ constexpr size_t kMaxBucketBytes = size_t(16) << 30;  // deferred bucket table b
 constexpr int64_t kDefaultChunk = 128;                // synapses per delivery task
 constexpr int64_t kMaxChunks = 64;                    // tasks per (spike, delay) segment
 constexpr int32_t kPersistentSteps = 1024;            // steps per cooperative launch
+constexpr int32_t kTileSteps = 4096;                  // of the tiled group (its prologue reads max delay steps)
 
 inline int bits_for(int64_t n)
 {
@@ -125,6 +127,12 @@ struct mgc_sim {
     size_t window_smem[2] = {0, 0};   // its dynamic shared memory [window > 4]: the delivery prefixes
     int acc_buffers = 4;              // accumulator buffers allocated (8 for a minimum delay >= 5)
     int group_grid1 = 1;              // minimum delay 1: the step group's grid
+    mgc::TileArgs tile{};             // tiled step group (tile.cuh): its layout, when the network
+    bool tile_ok = false;             //   qualifies (build_tiles),
+    bool tile_on = false;             //   whether steps run in it (by default; an explicit step-group
+                                      //   mode or the autotuner may take another form)
+    bool tile_one = false;            //   one delay, fp32 sums: 16-bit records
+    size_t tile_smem = 0;             //   its dynamic shared memory
     int32_t fx_shift = 0;             // fixed-point shift the builder picked for this network's weights
     bool hetero = false;              // some neuron receives unequal weights of one sign
     int32_t sched_mode_h = 0;         // host mirrors of what decides the graph's shape
@@ -180,6 +188,9 @@ struct mgc_sim {
 
 namespace mgc {
 
+// One attribute of the device (cudaGetDeviceProperties reads them all: 5 ms a call).
+mgc_status device_attr(cudaDeviceAttr attr, int device, int* value);
+
 // Temporary device buffer freed on scope exit.
 struct DevTmp {
     void* p = nullptr;
@@ -201,6 +212,7 @@ mgc_status tmp_alloc(DevTmp& t, T** p, size_t count)
 using StepKernel = void (*)(StepArgs);
 using GroupKernel = void (*)(StepArgs, int32_t);
 using WindowKernel = void (*)(StepArgs, int32_t, int32_t);
+using TileKernel = void (*)(StepArgs, TileArgs, int32_t);
 
 StepKernel neuron_kernel(const mgc_sim* s);
 StepKernel deliver_kernel(const mgc_sim* s);
@@ -216,6 +228,8 @@ GroupKernel pipe_kernel(const mgc_sim* s, int v);
 // The windowed step group of variant v: for windows of up to 4 steps, or
 // (wide) of up to 8; with pull steps (mgc_set_pull) or without.
 WindowKernel window_kernel(const mgc_sim* s, int v, bool wide, bool pull);
+// The tiled step group of this network (tile.cu).
+TileKernel tile_kernel(const mgc_sim* s);
 // The scheduler's decision kernel (sched.cu).
 const void* sched_decide_kernel();
 
@@ -246,6 +260,11 @@ int32_t fx_shift_rule(double bound, int min_exp, bool exact);
 mgc_status build_in_rows(mgc_sim* s);
 // Frees them again (pull steps off; the stream idle first).
 void release_in_rows(mgc_sim* s);
+// The tiled step group's synapses and buffers, when the network qualifies for
+// it (tile.cu); built again when the accumulation changes.
+mgc_status build_tiles(mgc_sim* s);
+// In-place exclusive scan of count + 1 entries (the last becomes the total).
+mgc_status scan_offsets(uint32_t* v, int64_t count, cudaStream_t st);
 // Segments of up to `gap` synapses cut into chunks of about `target`.
 void set_chunking(StepArgs& a, int64_t gap, int64_t target);
 

@@ -1,0 +1,267 @@
+// The tiled step group's host side: which networks take it, the synapses cut
+// by tile, and the kernel instantiations.
+#include "sim.h"
+
+namespace mgc {
+namespace {
+
+constexpr int kTileRowBlock = 256;
+constexpr int kMaxTiles = 256;
+// Above this many neurons, networks with fewer than 4 records a segment keep the
+// other step groups: every tile looks up a segment per spike, and at 200,000
+// neurons with 2 records a segment a driven step took 9.3 us against 5.8 for
+// the windowed group (a quiet one 2.4 against 3.2); at 100,000 neurons with 0.7
+// the tiles are the faster form on both loads (1.1 / 3.7 against 2.6 / 4.2).
+constexpr int kTileThinNeurons = 1 << 17;
+
+// Records per vector.
+__host__ __device__ constexpr int vec_records(bool fx, bool one) { return !fx && one ? 4 : 2; }
+
+// Vectors of every (source, tile) segment, one block per source row at a time;
+// with fp32 sums also each neuron's weight per sign, its in-degree, the
+// smallest and largest weight word per sign, and whether some source has
+// synapses of both signs (wstat[5]).
+template <bool FX, bool ONE>
+__global__ void __launch_bounds__(kTileRowBlock) k_tile_count(const int64_t* row_ptr, const uint2* syn, int32_t n_src,
+                                                              int32_t T, uint32_t tmask, uint32_t* off, float* we,
+                                                              float* wi, uint32_t* indeg, uint32_t* wstat)
+{
+    __shared__ uint32_t cnt[kMaxTiles];
+    constexpr uint32_t V = vec_records(FX, ONE);
+    uint32_t st[4] = {0xffffffffu, 0u, 0xffffffffu, 0u};  // exc min, max, inh min, max (words)
+    for (int64_t row = blockIdx.x; row < n_src; row += gridDim.x) {
+        const int64_t b = row_ptr[row], e = row_ptr[row + 1];
+        const bool first_exc = !FX && b < e && as_f(syn[b].y) > 0.0f;
+        for (int t = threadIdx.x; t < T; t += blockDim.x) cnt[t] = 0;
+        __syncthreads();
+        for (int64_t p = b + threadIdx.x; p < e; p += blockDim.x) {
+            const uint2 w = syn[p];
+            const uint32_t tgt = w.x & tmask;
+            atomicAdd(cnt + (tgt >> 2) % (uint32_t)T, 1u);
+            if (!FX) {
+                const float x = as_f(w.y);
+                const int h = x > 0.0f ? 0 : 2;
+                if ((x > 0.0f) != first_exc) wstat[5] = 1u;
+                (x > 0.0f ? we : wi)[tgt] = x;
+                st[h] = min(st[h], w.y);
+                st[h + 1] = max(st[h + 1], w.y);
+                atomicAdd(indeg + tgt, 1u);
+            }
+        }
+        __syncthreads();
+        for (int t = threadIdx.x; t < T; t += blockDim.x) off[(size_t)row * T + t] = (cnt[t] + V - 1) / V;
+        __syncthreads();
+    }
+    if (!FX) {
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1)
+#pragma unroll
+            for (int h = 0; h < 4; h += 2) {
+                st[h] = min(st[h], __shfl_xor_sync(0xffffffffu, st[h], o));
+                st[h + 1] = max(st[h + 1], __shfl_xor_sync(0xffffffffu, st[h + 1], o));
+            }
+        if ((threadIdx.x & 31) == 0)
+            for (int h = 0; h < 4; h += 2) {
+                atomicMin(wstat + h, st[h]);
+                atomicMax(wstat + h + 1, st[h + 1]);
+            }
+    }
+}
+
+constexpr uint32_t kIndex = 0x7fffffffu;  // off: vector index, the source's sign above (ONE)
+
+// The records into their segments (their order inside a segment does not
+// matter: the sums are counts or integers), the last vector filled up.
+template <bool FX, bool ONE>
+__global__ void __launch_bounds__(kTileRowBlock) k_tile_fill(const int64_t* row_ptr, const uint2* syn, int32_t n_src,
+                                                             int32_t T, uint32_t tmask, int tbits, int32_t nl,
+                                                             uint32_t* off, void* rec)
+{
+    __shared__ uint32_t pos[kMaxTiles];
+    constexpr uint32_t V = vec_records(FX, ONE);
+    auto put = [&](uint32_t at, uint32_t local, uint32_t d, uint32_t w, bool inh) {
+        if (FX)
+            reinterpret_cast<uint2*>(rec)[at] = make_uint2(local | (d << 16), w);
+        else if (ONE)
+            reinterpret_cast<uint16_t*>(rec)[at] = (uint16_t)(4u * local);
+        else
+            reinterpret_cast<uint32_t*>(rec)[at] = local | (d << 16) | (inh ? 0x80000000u : 0u);
+    };
+    for (int64_t row = blockIdx.x; row < n_src; row += gridDim.x) {
+        const int64_t b = row_ptr[row], e = row_ptr[row + 1];
+        for (int t = threadIdx.x; t < T; t += blockDim.x) pos[t] = (off[(size_t)row * T + t] & kIndex) * V;
+        __syncthreads();
+        for (int64_t p = b + threadIdx.x; p < e; p += blockDim.x) {
+            const uint2 w = syn[p];
+            const uint32_t tgt = w.x & tmask;
+            const uint32_t g = tgt >> 2, q = g / (uint32_t)T;
+            const uint32_t at = atomicAdd(pos + (g - q * (uint32_t)T), 1u);
+            put(at, (q << 2) + (tgt & 3u), w.x >> tbits, w.y, !(as_f(w.y) > 0.0f));
+        }
+        __syncthreads();
+        const uint32_t sign = ONE && b < e && !(as_f(syn[b].y) > 0.0f) ? ~kIndex : 0u;
+        for (int t = threadIdx.x; t < T; t += blockDim.x) {
+            // (the next entry may belong to another block's row, which sets only its top bit)
+            const uint32_t end = (*(volatile uint32_t*)(off + (size_t)row * T + t + 1) & kIndex) * V;
+            for (uint32_t at = pos[t]; at < end; ++at) put(at, ONE ? (uint32_t)nl : 0u, 0x7fffu, 0u, false);
+            if (sign) off[(size_t)row * T + t] |= sign;
+        }
+        __syncthreads();
+    }
+}
+
+__global__ void k_max_u32(const uint32_t* v, int64_t n, uint32_t* out)
+{
+    uint32_t m = 0;
+    GRID_STRIDE(i, n) m = max(m, v[i]);
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(out, m);
+}
+
+// chain[h][k]: k additions of the sign's weight from zero.
+__global__ void k_chain(const uint32_t* wstat, float* chain)
+{
+    const int h = threadIdx.x;
+    if (h >= 2) return;
+    const float w = as_f(wstat[2 * h]);
+    float v = 0.0f;
+    for (int k = 0; k < kTileTable; ++k) {
+        chain[h * kTileTable + k] = v;
+        v = fadd_ftz(v, w);
+    }
+}
+
+template <bool FX, bool ONE>
+static TileKernel tile_of(bool cur)
+{
+    return cur ? k_tile<true, FX, ONE> : k_tile<false, FX, ONE>;
+}
+
+}  // namespace
+
+TileKernel tile_kernel(const mgc_sim* s)
+{
+    if (s->a.fx) return tile_of<true, false>(s->a.has_cur);
+    return s->tile_one ? tile_of<false, true>(s->a.has_cur) : tile_of<false, false>(s->a.has_cur);
+}
+
+void release_tiles(mgc_sim* s)
+{
+    TileArgs& t = s->tile;
+    for (const void* p : {(const void*)t.off, t.rec, (const void*)t.we, (const void*)t.wi, (const void*)t.chain,
+                          (const void*)t.list, (const void*)t.mail, (const void*)t.cnt})
+        if (p) s->release(const_cast<void*>(p));
+    t = TileArgs{};
+    s->tile_ok = s->tile_on = false;
+}
+
+mgc_status build_tiles(mgc_sim* s)
+{
+    StepArgs& a = s->a;
+    release_tiles(s);
+    if (!a.deferred || s->partition || s->S <= 0 || (s->hetero && !a.fx) || s->dmax > kTileMaxDelay) return MGC_OK;
+    int sms = 0, optin = 0;
+    CKS(device_attr(cudaDevAttrMultiProcessorCount, s->device, &sms));
+    CKS(device_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device, &optin));
+    sms = std::min(sms, kMaxTiles);
+    const bool fx = a.fx != 0, cur = a.has_cur != 0;
+    bool one = !fx && s->dmax == s->dmin;  // and one sign per source, checked below
+    const size_t room = (size_t)optin - 1024;  // (static shared memory)
+    const int64_t groups = a.ns / 4;
+    if (a.ns >= (1 << kTileStepShift)) return MGC_OK;
+    auto nl_of = [&](int T) { return (int64_t)((groups + T - 1) / T * 4); };
+    auto fits = [&](int T) {
+        const int64_t nl = nl_of(T);
+        return nl < (one ? 0x3fff : 0x10000) && tile_smem_bytes((int)nl, s->dmax, T, fx, cur, !fx) <= room;
+    };
+    int T = (int)std::max<int64_t>(1, std::min<int64_t>({(int64_t)sms, groups, 2 * s->S / s->n}));
+    while (T < sms && !fits(T)) ++T;
+    const int64_t avg = s->S / ((int64_t)s->n * T);  // records per segment
+    if (!fits(T) || 2 * s->S / T < s->n || (avg < 4 && s->n > kTileThinNeurons)) return MGC_OK;
+    const size_t vec_bytes = fx ? 16 : 8;
+    // at most one vector in each segment is not full
+    const size_t most = ((size_t)s->S / 2 + (size_t)s->n * T) * vec_bytes;
+    const int W = std::min(kTileWindow, s->dmin);
+    const size_t need = most + ((size_t)s->n * T + 1) * 4 + 2 * (size_t)W * nl_of(T) * T * 4 + 16 * (size_t)a.ns;
+    // offsets in vectors, and in records while they are filled
+    if ((int64_t)s->n * T + 1 > (int64_t)0x7fffffff || most / vec_bytes > kIndex / 2) return MGC_OK;
+    size_t free_b = 0, total_b = 0;
+    CK(cudaMemGetInfo(&free_b, &total_b));
+    if (need > free_b / 2) return MGC_OK;
+    TileArgs& t = s->tile;
+    t.T = T;
+    t.nl = (int32_t)nl_of(T);
+    t.stride = tile_stride(t.nl);
+    t.R = s->dmax;
+    t.W = W;
+    t.dmin = s->dmin;
+    t.dmax = s->dmax;
+    t.ahead = s->fused ? 1 : 0;
+    uint32_t* off;
+    float *we = nullptr, *wi = nullptr, *chain = nullptr;
+    CKS(s->alloc(&off, (size_t)s->n * T + 1, false));
+    t.off = off;
+    CKS(s->alloc(&t.list, 2 * (size_t)T * t.nl * W, false));
+    CKS(s->alloc(&t.mail, 2 * (size_t)T * T));
+    t.epoch = 1;
+    CKS(s->alloc(&t.cnt, 4 * kTileWindow));
+    DevTmp t_deg, t_stat;
+    uint32_t *indeg = nullptr, *wstat = nullptr;
+    if (!fx) {
+        CKS(s->alloc(&we, a.ns));
+        t.we = we;
+        CKS(s->alloc(&wi, a.ns));
+        t.wi = wi;
+        CKS(s->alloc(&chain, 2 * kTileTable, false));
+        t.chain = chain;
+        CKS(tmp_alloc(t_deg, &indeg, a.ns));
+        CKS(tmp_alloc(t_stat, &wstat, 6));
+        const uint32_t init[6] = {0xffffffffu, 0u, 0xffffffffu, 0u, 0u, 0u};
+        CK(cudaMemsetAsync(indeg, 0, 4 * (size_t)a.ns, s->stream));
+        CK(cudaMemcpyAsync(wstat, init, sizeof(init), cudaMemcpyHostToDevice, s->stream));
+    }
+    const int grid = (int)std::min<int64_t>(s->n, (int64_t)sms * 8);
+    uint32_t h[6] = {};
+    auto count = [&]() -> mgc_status {
+        auto k = fx ? k_tile_count<true, false> : (one ? k_tile_count<false, true> : k_tile_count<false, false>);
+        k<<<grid, kTileRowBlock, 0, s->stream>>>(a.row_ptr, a.syn, s->n, T, a.tmask, off, we, wi, indeg, wstat);
+        CKS(scan_offsets(off, (int64_t)s->n * T, s->stream));
+        if (!fx) {
+            k_max_u32<<<grid_for(a.ns), 256, 0, s->stream>>>(indeg, a.ns, wstat + 4);
+            k_chain<<<1, 32, 0, s->stream>>>(wstat, chain);
+            CK(cudaMemcpyAsync(h, wstat, sizeof(h), cudaMemcpyDeviceToHost, s->stream));
+        }
+        CK(cudaMemcpyAsync(&t.n_vec, off + (size_t)s->n * T, 4, cudaMemcpyDeviceToHost, s->stream));
+        CK(cudaStreamSynchronize(s->stream));
+        return MGC_OK;
+    };
+    CKS(count());
+    if (one && h[5]) {  // a source with synapses of both signs: a sign in every record
+        one = false;
+        CK(cudaMemsetAsync(indeg, 0, 4 * (size_t)a.ns, s->stream));
+        CKS(count());
+    }
+    if (!fx) {
+        if (h[4] > 0xffffu) {  // a step's count of one sign might not fit its half word
+            release_tiles(s);
+            return MGC_OK;
+        }
+        t.table = (h[0] >= h[1] && h[2] >= h[3]) ? 1 : 0;
+    }
+    t.lanes_log2 = avg < 10 * vec_records(fx, one) ? 0 : 2;
+    char* rec;
+    CKS(s->alloc(&rec, std::max<size_t>(1, t.n_vec) * vec_bytes, false));
+    t.rec = rec;
+    auto fill = fx ? k_tile_fill<true, false> : (one ? k_tile_fill<false, true> : k_tile_fill<false, false>);
+    fill<<<grid, kTileRowBlock, 0, s->stream>>>(a.row_ptr, a.syn, s->n, T, a.tmask, a.tbits, t.nl, off, rec);
+    CK(cudaGetLastError());
+    s->tile_one = one;
+    s->tile_smem = tile_smem_bytes(t.nl, t.R, T, fx, cur, t.table != 0);
+    CK(cudaFuncSetAttribute((const void*)tile_kernel(s), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)s->tile_smem));
+    s->tile_ok = s->tile_on = true;
+    return MGC_OK;
+}
+
+}  // namespace mgc

@@ -160,6 +160,7 @@ mgc_status mgc_set_persistent(mgc_sim* s, int32_t mode)
         s->sched_graph = false;
     }
     s->persistent = mode;
+    s->tile_on = false;  // the caller's form, not the builder's choice
     return MGC_OK;
 }
 
@@ -202,9 +203,8 @@ mgc_status mgc_autotune(mgc_sim* s, int64_t steps_per_trial, mgc_tune_report* re
     if (s->partition) return fail(MGC_ERR_INVALID, "partition handles run steps only between exchanges (mgc_run)");
     CK(cudaSetDevice(s->device));
     memset(rep, 0, sizeof(*rep));
-    cudaDeviceProp prop;
-    CK(cudaGetDeviceProperties(&prop, s->device));
-    const int sms = prop.multiProcessorCount;
+    int sms = 0;
+    CKS(device_attr(cudaDevAttrMultiProcessorCount, s->device, &sms));
     int occ = 1, occ_min = 1;
     if (s->fused) {
         occ_min = 2;  // the two instantiations of the fused kernel
@@ -233,6 +233,7 @@ mgc_status mgc_autotune(mgc_sim* s, int64_t steps_per_trial, mgc_tune_report* re
     if (!s->a.deferred)
         for (int g : {16, 37, 74}) cands.push_back({0, 1, g});
     const int64_t steps = (steps_per_trial + kGraphSteps - 1) / kGraphSteps * kGraphSteps;
+    s->tile_on = false;
     s->persistent = 0;  // the shapes are timed as graphs of single-step kernels, step groups after
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     CK(cudaEventCreate(&e0));
@@ -346,6 +347,32 @@ mgc_status mgc_autotune(mgc_sim* s, int64_t steps_per_trial, mgc_tune_report* re
         if (st == MGC_OK) st = mgc_sync(s);
     }
     if (pull_ok && st == MGC_OK) st = mgc_set_pull(s, 0);
+    // the tiled step group, where the network has its layout: it runs in the
+    // place of the builder's default step-group mode
+    if (s->tile_ok && st == MGC_OK && !sched_wanted(s)) {
+        s->persistent = s->dmin >= 4 ? 2 : 1;
+        s->tile_on = true;
+        st = mgc_run(s, kGraphSteps);
+        if (st == MGC_OK) {
+            cudaEventRecord(e0, s->stream);
+            st = mgc_run(s, steps);
+            cudaEventRecord(e1, s->stream);
+        }
+        float ms = 0.f;
+        if (st == MGC_OK && cudaEventSynchronize(e1) == cudaSuccess && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess) {
+            const double per = (double)ms / (double)steps;
+            rep->trials += 1;
+            if (per < best && s->tile_on) {
+                best = per;
+                rep->persistent = s->persistent;
+                best_window = window0;
+                best_pull = 0;
+            } else {
+                s->tile_on = false;
+            }
+        }
+        if (st == MGC_OK) st = mgc_sync(s);
+    }
     s->persistent = rep->persistent;
     s->window = best_window;
     rep->window = s->fused ? s->window : 0;
