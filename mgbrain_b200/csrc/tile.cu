@@ -18,13 +18,13 @@ constexpr int kTileThinNeurons = 1 << 17;
 __host__ __device__ constexpr int vec_records(bool fx, bool one) { return !fx && one ? 4 : 2; }
 
 // Vectors of every (source, tile) segment, one block per source row at a time;
-// with fp32 sums also each neuron's weight per sign, its in-degree, the
-// smallest and largest weight word per sign, and whether some source has
-// synapses of both signs (wstat[5]).
+// with fp32 sums also each neuron's in-degree, the smallest and largest weight
+// word per sign, and whether some source has synapses of both signs
+// (wstat[5]).
 template <bool FX, bool ONE>
 __global__ void __launch_bounds__(kTileRowBlock) k_tile_count(const int64_t* row_ptr, const uint2* syn, int32_t n_src,
-                                                              int32_t T, uint32_t tmask, uint32_t* off, float* we,
-                                                              float* wi, uint32_t* indeg, uint32_t* wstat)
+                                                              int32_t T, uint32_t tmask, uint32_t* off,
+                                                              uint32_t* indeg, uint32_t* wstat)
 {
     __shared__ uint32_t cnt[kMaxTiles];
     constexpr uint32_t V = vec_records(FX, ONE);
@@ -42,7 +42,6 @@ __global__ void __launch_bounds__(kTileRowBlock) k_tile_count(const int64_t* row
                 const float x = as_f(w.y);
                 const int h = x > 0.0f ? 0 : 2;
                 if ((x > 0.0f) != first_exc) wstat[5] = 1u;
-                (x > 0.0f ? we : wi)[tgt] = x;
                 st[h] = min(st[h], w.y);
                 st[h + 1] = max(st[h + 1], w.y);
                 atomicAdd(indeg + tgt, 1u);
@@ -107,6 +106,26 @@ __global__ void __launch_bounds__(kTileRowBlock) k_tile_fill(const int64_t* row_
             if (sign) off[(size_t)row * T + t] |= sign;
         }
         __syncthreads();
+    }
+}
+
+// Each neuron's weight per sign: the network's (word of each sign), or from its
+// synapses.
+__global__ void k_tile_weights(const uint2* syn, int64_t S, uint32_t tmask, float* we, float* wi)
+{
+    GRID_STRIDE(p, S)
+    {
+        const uint2 w = syn[p];
+        const float x = as_f(w.y);
+        (x > 0.0f ? we : wi)[w.x & tmask] = x;
+    }
+}
+__global__ void k_tile_weight(const uint32_t* wstat, int64_t n, float* we, float* wi)
+{
+    GRID_STRIDE(i, n)
+    {
+        we[i] = as_f(wstat[0]);
+        wi[i] = as_f(wstat[2]);
     }
 }
 
@@ -225,7 +244,7 @@ mgc_status build_tiles(mgc_sim* s)
     uint32_t h[6] = {};
     auto count = [&]() -> mgc_status {
         auto k = fx ? k_tile_count<true, false> : (one ? k_tile_count<false, true> : k_tile_count<false, false>);
-        k<<<grid, kTileRowBlock, 0, s->stream>>>(a.row_ptr, a.syn, s->n, T, a.tmask, off, we, wi, indeg, wstat);
+        k<<<grid, kTileRowBlock, 0, s->stream>>>(a.row_ptr, a.syn, s->n, T, a.tmask, off, indeg, wstat);
         CKS(scan_offsets(off, (int64_t)s->n * T, s->stream));
         if (!fx) {
             k_max_u32<<<grid_for(a.ns), 256, 0, s->stream>>>(indeg, a.ns, wstat + 4);
@@ -248,6 +267,10 @@ mgc_status build_tiles(mgc_sim* s)
             return MGC_OK;
         }
         t.table = (h[0] >= h[1] && h[2] >= h[3]) ? 1 : 0;
+        if (t.table)
+            k_tile_weight<<<grid_for(a.ns), 256, 0, s->stream>>>(wstat, a.ns, we, wi);
+        else
+            k_tile_weights<<<grid_for(s->S), 256, 0, s->stream>>>(a.syn, s->S, a.tmask, we, wi);
     }
     t.lanes_log2 = avg < 10 * vec_records(fx, one) ? 0 : 2;
     char* rec;
