@@ -561,6 +561,7 @@ mgc_status finish_build(mgc_sim* s)
     a.M = s->M;
     CKS(launch_shapes(s));
     CKS(build_tiles(s));
+    CKS(init_readout(s));
     CK(cudaStreamSynchronize(s->stream));
     return MGC_OK;
 }

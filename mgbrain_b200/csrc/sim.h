@@ -88,6 +88,16 @@ struct mgc_sim {
         cudaEvent_t ev = nullptr;
     };
     RasterStage stages[2];
+    // readout: the raster's running sums and meta words, the sort's launch shape
+    // (and its bitmaps, when they don't fit in shared memory), one buffer for a
+    // small network's state
+    int64_t *raster_off = nullptr, *raster_meta = nullptr;
+    int64_t sort_words = 0;
+    int sort_grid = 1;
+    size_t sort_smem = 0;
+    uint32_t* sort_bitmap = nullptr;
+    uint32_t* state_buf = nullptr;
+    std::vector<uint32_t> state_host;
     int stage_head = 0, staged = 0;  // oldest outstanding stage, and how many
     cudaStream_t copy_stream = nullptr;
     int32_t pending = 0;     // partition: steps run since the last spike import
@@ -265,6 +275,8 @@ void release_in_rows(mgc_sim* s);
 mgc_status build_tiles(mgc_sim* s);
 // In-place exclusive scan of count + 1 entries (the last becomes the total).
 mgc_status scan_offsets(uint32_t* v, int64_t count, cudaStream_t st);
+// The readout's buffers (readout.cu).
+mgc_status init_readout(mgc_sim* s);
 // Segments of up to `gap` synapses cut into chunks of about `target`.
 void set_chunking(StepArgs& a, int64_t gap, int64_t target);
 
