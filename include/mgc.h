@@ -449,7 +449,8 @@ mgc_status mgc_autotune_rewind(mgc_sim* sim, int64_t steps_per_trial, mgc_tune_r
  * whose state fits on the chip runs the tiled step group in the place of that
  * mode (one block per SM keeps its neurons' state and inputs in shared memory
  * and delivers every spike to its own targets from a copy of the synapses cut
- * by block); a mode set here runs as described.  If the device cannot keep all blocks of a group resident, the
+ * by block), and other networks run the windowed group in the place of mode 2;
+ * a mode set here runs as described.  If the device cannot keep all blocks of a group resident, the
  * call falls back to 0.  Results are the same in every mode; while a schedule mode other than
  * static, recording or calibration is on, graphs are used.  All waits are
  * bounded (a time-out makes mgc_sync return MGC_ERR_CUDA).  No reference

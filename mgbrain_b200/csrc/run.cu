@@ -76,9 +76,23 @@ namespace mgc {
 // the barrier per step, for a minimum delay below 4) in its place.
 int graph_group_mode(const mgc_sim* s, int p) { return p == 3 ? (s->dmin >= 4 ? 2 : 1) : p; }
 
+// The builder's choice runs as the windowed group where the pipelined one
+// (minimum delay >= 4) would run: it gives the same bits and is the faster of
+// the two at every measured size and load (1.1e9 synapses quiet 4.9 against
+// 8.6 us per step, driven 49 against 57; 1e5 neurons 2.6 against 5.6).  Not
+// with fp32 sums of unequal weights of one sign (a caller's choice), whose
+// last bits follow the order of the additions, and not for partitions, whose
+// windows of minimum delay - 1 steps are a launch each.
+int group_mode(const mgc_sim* s)
+{
+    const bool windowed = s->auto_form && s->persistent == 2 && !s->partition && !(s->hetero && !s->a.fx);
+    return windowed ? 3 : s->persistent;
+}
+
 int32_t wanted_acc_mask(const mgc_sim* s)
 {
-    const bool wide = s->acc_buffers == kAccBuffersWide && s->persistent == 3 && s->window > kAccBuffers;
+    const bool wide = s->acc_buffers == kAccBuffersWide && group_mode(s) == 3 && !s->tile_on &&
+                      s->window > kAccBuffers;
     return wide && !sched_wanted(s) ? kAccBuffersWide - 1 : kAccBuffers - 1;
 }
 
@@ -289,7 +303,7 @@ mgc_status mgc_run(mgc_sim* s, int64_t steps)
     if (s->persistent && s->a.deferred && !sched_wanted(s)) {
         // one cooperative launch per group: every block resident, a grid
         // barrier between steps (or the pipelined arrive/wait) instead of a launch
-        const int p = s->persistent, v = s->fused_variant;
+        const int p = group_mode(s), v = s->fused_variant;  // (where the tiled group does not run)
         while (left > 0) {
             int32_t n = (int32_t)std::min<int64_t>(left, s->tile_on ? kTileSteps : kPersistentSteps);
             // the schedule trace only while the scheduler's graph runs
@@ -306,6 +320,7 @@ mgc_status mgc_run(mgc_sim* s, int64_t steps)
                 if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
                     cudaGetLastError();  // not all resident here: the other step groups
                     s->tile_on = false;
+                    CKS(set_acc_mask(s, wanted_acc_mask(s), true));
                     continue;
                 }
                 if (e == cudaSuccess) s->tile.epoch += (uint32_t)((n + s->tile.W - 1) / s->tile.W + 1);  // windows, the end
@@ -331,6 +346,7 @@ mgc_status mgc_run(mgc_sim* s, int64_t steps)
                 // device): fall back to the graphs of single-step kernels
                 cudaGetLastError();
                 s->persistent = 0;
+                s->auto_form = false;
                 break;
             }
             CK(e);

@@ -132,6 +132,7 @@ struct mgc_sim {
     int persistent = 0;               // fused method as cooperative step groups: 1 barrier per
                                       // step, 2 pipelined (min delay >= 4), 3 windowed
     int group_grid_v[2][2] = {{1, 1}, {1, 1}};  // [persistent-1][variant] co-resident grids
+    bool auto_form = true;            // no caller and no autotuner has chosen the step-group form
     int window = 1;                   // steps per window of the windowed group (<= min delay, <= 8)
     int window_grid_v[2][2] = {{1, 1}, {1, 1}};  // its co-resident grids [window > 4][variant]
     size_t window_smem[2] = {0, 0};   // its dynamic shared memory [window > 4]: the delivery prefixes
@@ -287,6 +288,9 @@ mgc_status build_graph(mgc_sim* s);
 mgc_status build_sched_graph(mgc_sim* s);
 bool sched_wanted(const mgc_sim* s);
 mgc_status refresh_graph(mgc_sim* s);
+// The step-group mode the next steps run in, outside the scheduler's graph and
+// the tiled group.
+int group_mode(const mgc_sim* s);
 // The step-group mode the scheduler's graph runs for mode p.
 int graph_group_mode(const mgc_sim* s, int p);
 // The accumulator cycle the next steps run with: 7 (eight buffers) while

@@ -160,7 +160,7 @@ mgc_status mgc_set_persistent(mgc_sim* s, int32_t mode)
         s->sched_graph = false;
     }
     s->persistent = mode;
-    s->tile_on = false;  // the caller's form, not the builder's choice
+    s->tile_on = s->auto_form = false;  // the caller's form, not the builder's choice
     return MGC_OK;
 }
 
@@ -233,7 +233,7 @@ mgc_status mgc_autotune(mgc_sim* s, int64_t steps_per_trial, mgc_tune_report* re
     if (!s->a.deferred)
         for (int g : {16, 37, 74}) cands.push_back({0, 1, g});
     const int64_t steps = (steps_per_trial + kGraphSteps - 1) / kGraphSteps * kGraphSteps;
-    s->tile_on = false;
+    s->tile_on = s->auto_form = false;
     s->persistent = 0;  // the shapes are timed as graphs of single-step kernels, step groups after
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     CK(cudaEventCreate(&e0));
