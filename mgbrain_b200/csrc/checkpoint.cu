@@ -134,6 +134,7 @@ mgc_status mgc_checkpoint_load(mgc_sim* s, const void* buf, int64_t bytes)
         CK(cudaMemcpy(&ev, s->a.events, 8, cudaMemcpyDeviceToHost));
         CK(cudaMemcpy(s->a.ev_mark, &ev, 8, cudaMemcpyHostToDevice));
     }
+    s->tile_stale = s->stdp && s->tile_ok;  // the weights are the checkpoint's
     s->ahead = h.ahead != 0;
     s->pending = 0;  // a partition's checkpoint is taken between exchanges
     CKS(set_acc_mask(s, h.acc_mask, false));  // the restored buffers' cycle

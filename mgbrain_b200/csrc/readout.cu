@@ -246,6 +246,9 @@ mgc_status init_readout(mgc_sim* s)
         CKS(s->alloc(&s->state_buf, 6 * (size_t)s->n, false));
         s->state_host.resize(6 * (size_t)s->n);
     }
+    // weights that change are read again and again (cudaMalloc and cudaFree in
+    // the call took up to 600 ms on a busy driver)
+    if (s->stdp && s->S > 0) CKS(s->alloc(&s->weights_buf, s->S, false));
     if (!s->a.record) return MGC_OK;
     CKS(s->alloc(&s->raster_meta, 5));
     CKS(s->alloc(&s->raster_off, (size_t)s->raster_steps_cap + 1, false));
@@ -389,8 +392,8 @@ mgc_status mgc_read_weights(mgc_sim* s, float* weight)
     const uint2* src_words = s->a.pull ? s->a.in_ent : s->a.syn;  // the pull method's live weights
     const int64_t* src_idx = s->a.pull ? s->in_syn64 : s->csr_syn64;
     DevTmp t;
-    float* out;
-    CKS(tmp_alloc(t, &out, s->S));
+    float* out = s->weights_buf;
+    if (!out) CKS(tmp_alloc(t, &out, s->S));
     k_weights_out<<<grid_for(s->S), 256, 0, s->stream>>>(src_words, src_idx, s->S, out);
     CK(cudaGetLastError());
     s->launches += 1;

@@ -300,7 +300,7 @@ mgc_status mgc_run(mgc_sim* s, int64_t steps)
         CKS(enqueue_step(s));  // catches up the delivery, leaves ahead = true
         --left;
     }
-    if (s->persistent && s->a.deferred && !sched_wanted(s)) {
+    if (((s->persistent && s->a.deferred) || s->tile_on) && !sched_wanted(s)) {
         // one cooperative launch per group: every block resident, a grid
         // barrier between steps (or the pipelined arrive/wait) instead of a launch
         const int p = group_mode(s), v = s->fused_variant;  // (where the tiled group does not run)
@@ -314,12 +314,14 @@ mgc_status mgc_run(mgc_sim* s, int64_t steps)
                 CK(cudaMemsetAsync(s->a.bar, 0, 4 * sizeof(unsigned int), s->stream));  // clean barriers
             cudaError_t e;
             if (s->tile_on) {
+                CKS(refresh_tiles(s));
                 void* targs[] = {&ga, &s->tile, &n};
                 e = cudaLaunchCooperativeKernel((const void*)tile_kernel(s), dim3(s->tile.T), dim3(kTileThreads),
                                                 targs, s->tile_smem, s->stream);
                 if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
                     cudaGetLastError();  // not all resident here: the other step groups
                     s->tile_on = false;
+                    if (!s->a.deferred) break;
                     CKS(set_acc_mask(s, wanted_acc_mask(s), true));
                     continue;
                 }
@@ -355,6 +357,7 @@ mgc_status mgc_run(mgc_sim* s, int64_t steps)
         }
         if (left == 0) return MGC_OK;
     }
+    if (s->stdp && s->tile_ok && left > 0) s->tile_stale = true;
     if (left >= kGraphSteps) {
         if (!s->graph) CKS(sched_wanted(s) ? build_sched_graph(s) : build_graph(s));
         while (left >= s->graph_steps) {

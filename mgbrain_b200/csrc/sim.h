@@ -96,6 +96,7 @@ struct mgc_sim {
     int sort_grid = 1;
     size_t sort_smem = 0;
     uint32_t* sort_bitmap = nullptr;
+    float* weights_buf = nullptr;    // plastic networks: the weights in list order
     uint32_t* state_buf = nullptr;
     std::vector<uint32_t> state_host;
     int stage_head = 0, staged = 0;  // oldest outstanding stage, and how many
@@ -142,6 +143,7 @@ struct mgc_sim {
     bool tile_ok = false;             //   qualifies (build_tiles),
     bool tile_on = false;             //   whether steps run in it (by default; an explicit step-group
                                       //   mode or the autotuner may take another form)
+    bool tile_stale = false;          //   STDP: other forms changed the weights since its last step
     bool tile_one = false;            //   one delay, fp32 sums: 16-bit records
     size_t tile_smem = 0;             //   its dynamic shared memory
     int32_t fx_shift = 0;             // fixed-point shift the builder picked for this network's weights
@@ -274,6 +276,8 @@ void release_in_rows(mgc_sim* s);
 // The tiled step group's synapses and buffers, when the network qualifies for
 // it (tile.cu); built again when the accumulation changes.
 mgc_status build_tiles(mgc_sim* s);
+// STDP: the tiles' weights brought up to date before they run (enqueued).
+mgc_status refresh_tiles(mgc_sim* s);
 // In-place exclusive scan of count + 1 entries (the last becomes the total).
 mgc_status scan_offsets(uint32_t* v, int64_t count, cudaStream_t st);
 // The readout's buffers (readout.cu).

@@ -21,13 +21,12 @@ __host__ __device__ constexpr int vec_records(bool fx, bool one) { return !fx &&
 // with fp32 sums also each neuron's in-degree, the smallest and largest weight
 // word per sign, and whether some source has synapses of both signs
 // (wstat[5]).
-template <bool FX, bool ONE>
+template <bool FX, bool ONE, uint32_t V = vec_records(FX, ONE)>
 __global__ void __launch_bounds__(kTileRowBlock) k_tile_count(const int64_t* row_ptr, const uint2* syn, int32_t n_src,
                                                               int32_t T, uint32_t tmask, uint32_t* off,
                                                               uint32_t* indeg, uint32_t* wstat)
 {
     __shared__ uint32_t cnt[kMaxTiles];
-    constexpr uint32_t V = vec_records(FX, ONE);
     uint32_t st[4] = {0xffffffffu, 0u, 0xffffffffu, 0u};  // exc min, max, inh min, max (words)
     for (int64_t row = blockIdx.x; row < n_src; row += gridDim.x) {
         const int64_t b = row_ptr[row], e = row_ptr[row + 1];
@@ -109,6 +108,55 @@ __global__ void __launch_bounds__(kTileRowBlock) k_tile_fill(const int64_t* row_
     }
 }
 
+// Plastic networks: the records with their plastic flag and CSR position, and
+// the plastic synapses onto each local neuron counted.
+__global__ void __launch_bounds__(kTileRowBlock) k_tile_fill_stdp(const int64_t* row_ptr, const uint2* syn,
+                                                                  const uint8_t* plastic, int32_t n_src, int32_t T,
+                                                                  int32_t nl, uint32_t tmask, int tbits,
+                                                                  const uint32_t* off, uint2* rec, uint32_t* cpos,
+                                                                  uint32_t* in_cnt)
+{
+    __shared__ uint32_t pos[kMaxTiles];
+    for (int64_t row = blockIdx.x; row < n_src; row += gridDim.x) {
+        const int64_t b = row_ptr[row], e = row_ptr[row + 1];
+        for (int t = threadIdx.x; t < T; t += blockDim.x) pos[t] = off[(size_t)row * T + t];
+        __syncthreads();
+        for (int64_t p = b + threadIdx.x; p < e; p += blockDim.x) {
+            const uint2 w = syn[p];
+            const uint32_t tgt = w.x & tmask;
+            const uint32_t g = tgt >> 2, q = g / (uint32_t)T, t = g - q * (uint32_t)T;
+            const uint32_t local = (q << 2) + (tgt & 3u);
+            const bool pl = !plastic || plastic[p];
+            const uint32_t at = atomicAdd(pos + t, 1u);
+            rec[at] = make_uint2(local | ((w.x >> tbits) << 16) | (pl ? 0x80000000u : 0u), w.y);
+            cpos[at] = (uint32_t)p;
+            if (pl) atomicAdd(in_cnt + (size_t)t * nl + local, 1u);
+        }
+        __syncthreads();
+    }
+}
+
+// The incoming lists {source, record} of the plastic synapses (each synapse is
+// updated by itself, so their order does not matter); at: running places.
+__global__ void k_tile_in(const uint2* rec, const uint32_t* cpos, const int32_t* csr_src, const uint2* syn, int64_t S,
+                          int32_t T, int32_t nl, uint32_t tmask, uint32_t* at, uint2* in_ent)
+{
+    GRID_STRIDE(r, S)
+    {
+        const uint2 w = rec[r];
+        if (!(w.x >> 31)) continue;
+        const uint32_t p = cpos[r];
+        const uint32_t t = ((syn[p].x & tmask) >> 2) % (uint32_t)T;
+        in_ent[atomicAdd(at + (size_t)t * nl + (w.x & 0xffffu), 1u)] = make_uint2((uint32_t)csr_src[p], (uint32_t)r);
+    }
+}
+
+// The records' weights from the CSR, after other step forms changed it.
+__global__ void k_tile_refresh(const uint2* syn, const uint32_t* cpos, int64_t S, uint2* rec)
+{
+    GRID_STRIDE(r, S) rec[r].y = syn[cpos[r]].y;
+}
+
 // Each neuron's weight per sign: the network's (word of each sign), or from its
 // synapses.
 __global__ void k_tile_weights(const uint2* syn, int64_t S, uint32_t tmask, float* we, float* wi)
@@ -161,6 +209,7 @@ static TileKernel tile_of(bool cur)
 
 TileKernel tile_kernel(const mgc_sim* s)
 {
+    if (s->stdp) return s->a.has_cur ? k_tile_stdp<true> : k_tile_stdp<false>;
     if (s->a.fx) return tile_of<true, false>(s->a.has_cur);
     return s->tile_one ? tile_of<false, true>(s->a.has_cur) : tile_of<false, false>(s->a.has_cur);
 }
@@ -169,7 +218,8 @@ void release_tiles(mgc_sim* s)
 {
     TileArgs& t = s->tile;
     for (const void* p : {(const void*)t.off, t.rec, (const void*)t.we, (const void*)t.wi, (const void*)t.chain,
-                          (const void*)t.list, (const void*)t.mail, (const void*)t.cnt})
+                          (const void*)t.list, (const void*)t.mail, (const void*)t.cnt, (const void*)t.cpos,
+                          (const void*)t.in_off, (const void*)t.in_ent})
         if (p) s->release(const_cast<void*>(p));
     t = TileArgs{};
     s->tile_ok = s->tile_on = false;
@@ -179,7 +229,9 @@ mgc_status build_tiles(mgc_sim* s)
 {
     StepArgs& a = s->a;
     release_tiles(s);
-    if (!a.deferred || s->partition || s->S <= 0 || (s->hetero && !a.fx) || s->dmax > kTileMaxDelay) return MGC_OK;
+    const bool stdp = s->stdp && !a.deferred && !a.pull && a.fx;  // the ring method with STDP
+    if ((!a.deferred && !stdp) || s->partition || s->S <= 0 || (s->hetero && !a.fx) || s->dmax > kTileMaxDelay)
+        return MGC_OK;
     int sms = 0, optin = 0;
     CKS(device_attr(cudaDevAttrMultiProcessorCount, s->device, &sms));
     CKS(device_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device, &optin));
@@ -192,6 +244,7 @@ mgc_status build_tiles(mgc_sim* s)
     auto nl_of = [&](int T) { return (int64_t)((groups + T - 1) / T * 4); };
     auto fits = [&](int T) {
         const int64_t nl = nl_of(T);
+        if (stdp) return nl < 0x10000 && tile_stdp_bytes((int)nl, s->dmax, T, cur, s->n) <= room;
         return nl < (one ? 0x3fff : 0x10000) && tile_smem_bytes((int)nl, s->dmax, T, fx, cur, !fx) <= room;
     };
     int T = (int)std::max<int64_t>(1, std::min<int64_t>({(int64_t)sms, groups, 2 * s->S / s->n}));
@@ -201,8 +254,8 @@ mgc_status build_tiles(mgc_sim* s)
     const size_t vec_bytes = fx ? 16 : 8;
     // at most one vector in each segment is not full
     const size_t most = ((size_t)s->S / 2 + (size_t)s->n * T) * vec_bytes;
-    const int W = std::min(kTileWindow, s->dmin);
-    const size_t need = most + ((size_t)s->n * T + 1) * 4 + 2 * (size_t)W * nl_of(T) * T * 4 + 16 * (size_t)a.ns;
+    const int W = stdp ? 1 : std::min(kTileWindow, s->dmin);
+    const size_t need = most + (stdp ? 12 * (size_t)s->S : 0) + ((size_t)s->n * T + 1) * 4 + 2 * (size_t)W * nl_of(T) * T * 4 + 16 * (size_t)a.ns;
     // offsets in vectors, and in records while they are filled
     if ((int64_t)s->n * T + 1 > (int64_t)0x7fffffff || most / vec_bytes > kIndex / 2) return MGC_OK;
     size_t free_b = 0, total_b = 0;
@@ -243,7 +296,7 @@ mgc_status build_tiles(mgc_sim* s)
     const int grid = (int)std::min<int64_t>(s->n, (int64_t)sms * 8);
     uint32_t h[6] = {};
     auto count = [&]() -> mgc_status {
-        auto k = fx ? k_tile_count<true, false> : (one ? k_tile_count<false, true> : k_tile_count<false, false>);
+        auto k = stdp ? k_tile_count<true, false, 1> : fx ? k_tile_count<true, false> : (one ? k_tile_count<false, true> : k_tile_count<false, false>);
         k<<<grid, kTileRowBlock, 0, s->stream>>>(a.row_ptr, a.syn, s->n, T, a.tmask, off, indeg, wstat);
         CKS(scan_offsets(off, (int64_t)s->n * T, s->stream));
         if (!fx) {
@@ -273,6 +326,39 @@ mgc_status build_tiles(mgc_sim* s)
             k_tile_weights<<<grid_for(s->S), 256, 0, s->stream>>>(a.syn, s->S, a.tmask, we, wi);
     }
     t.lanes_log2 = avg < 10 * vec_records(fx, one) ? 0 : 2;
+    if (stdp) {
+        uint2 *srec, *in_ent;
+        uint32_t *cpos, *in_off;
+        const int64_t locals = (int64_t)T * t.nl;
+        CKS(s->alloc(&srec, s->S, false));
+        t.rec = srec;
+        CKS(s->alloc(&cpos, s->S, false));
+        t.cpos = cpos;
+        CKS(s->alloc(&in_off, locals + 1));
+        t.in_off = in_off;
+        DevTmp t_at;
+        uint32_t* at;
+        CKS(tmp_alloc(t_at, &at, locals + 1));
+        k_tile_fill_stdp<<<grid, kTileRowBlock, 0, s->stream>>>(a.row_ptr, a.syn, a.plastic, s->n, T, t.nl, a.tmask,
+                                                                a.tbits, off, srec, cpos, in_off);
+        CKS(scan_offsets(in_off, locals, s->stream));
+        uint32_t n_in = 0;
+        CK(cudaMemcpyAsync(&n_in, in_off + locals, 4, cudaMemcpyDeviceToHost, s->stream));
+        CK(cudaMemcpyAsync(at, in_off, 4 * (size_t)locals, cudaMemcpyDeviceToDevice, s->stream));
+        CK(cudaStreamSynchronize(s->stream));
+        CKS(s->alloc(&in_ent, n_in, false));
+        t.in_ent = in_ent;
+        k_tile_in<<<grid_for(s->S), 256, 0, s->stream>>>(srec, cpos, a.csr_src, a.syn, s->S, T, t.nl, a.tmask, at,
+                                                         in_ent);
+        CK(cudaGetLastError());
+        CK(cudaStreamSynchronize(s->stream));
+        s->tile_smem = tile_stdp_bytes(t.nl, t.R, T, cur, s->n);
+        CK(cudaFuncSetAttribute((const void*)tile_kernel(s), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)s->tile_smem));
+        s->tile_ok = s->tile_on = true;
+        s->tile_stale = false;
+        return MGC_OK;
+    }
     char* rec;
     CKS(s->alloc(&rec, std::max<size_t>(1, t.n_vec) * vec_bytes, false));
     t.rec = rec;
@@ -284,6 +370,17 @@ mgc_status build_tiles(mgc_sim* s)
     CK(cudaFuncSetAttribute((const void*)tile_kernel(s), cudaFuncAttributeMaxDynamicSharedMemorySize,
                             (int)s->tile_smem));
     s->tile_ok = s->tile_on = true;
+    return MGC_OK;
+}
+
+mgc_status refresh_tiles(mgc_sim* s)
+{
+    if (!s->tile_stale) return MGC_OK;
+    k_tile_refresh<<<grid_for(s->S), 256, 0, s->stream>>>(s->a.syn, s->tile.cpos, s->S,
+                                                           static_cast<uint2*>(const_cast<void*>(s->tile.rec)));
+    CK(cudaGetLastError());
+    s->launches += 1;
+    s->tile_stale = false;
     return MGC_OK;
 }
 

@@ -92,6 +92,10 @@ struct TileArgs {
     ulonglong2* mail;     // [2][T reader][T] headers {epoch << 32 | count, first spikes}
     uint32_t epoch;       // epoch of the launch's first window (they count on over the launches)
     int32_t* cnt;         // [4][kTileWindow] spikes of a window's steps; zero between launches
+    // plastic networks (k_tile_stdp): rec holds single records (off counts them)
+    const uint32_t* cpos;   // [S] CSR position of a record
+    const uint32_t* in_off; // [T*nl + 1] plastic synapses onto each local neuron, tile after tile:
+    const uint2* in_ent;    //   {source, record}
 };
 
 constexpr int kTileInline = 2;      // spikes a header carries
@@ -906,6 +910,269 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
         *a.done = 0;
         a.slots[0] = (int32_t)((slot0 + nsteps) % a.M);
         a.slots[1] = hs_of(s_end);
+        *a.step = s_end;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The same for the ring method with STDP (fixed-point sums): one step per
+// window, since a step's pushes read the weights that the spikes of the step
+// before changed.  A tile owns the synapses onto its neurons, so both sides of
+// STDP are its own work: its records of a spiking source are pushed and
+// depressed, the plastic records onto a spiking neuron of its own are
+// potentiated (those whose source spiked too belong to the first, as in
+// k_push_stdp), and no weight has two writers.  last_fired of the whole network
+// and the step's spikes as a bitmap are kept in shared memory by every block,
+// from the spike ids that the exchange brings.  A weight is written to its record
+// and to the CSR, which stays current for readers and the other step forms
+// (records are refreshed from it after those ran).  The launch takes over
+// the global ring's pending input and hands it back.
+//
+// Bound by the step's chain of dependent accesses: exchange, segment
+// offsets, records, and after a spike of its own the incoming list and its
+// weights.  784 -> 1,600 plastic network, 1.9e4 events a step: see DESIGN.
+// ---------------------------------------------------------------------------
+struct TileStdpSmem {
+    int32_t* lf;       // [n] last spike of every neuron
+    uint32_t* fired;   // [n/32] this step's spikes
+    uint32_t* in_off;  // [nl + 1] this tile's part of t.in_off
+};
+
+__host__ __device__ inline size_t tile_stdp_bytes(int nl, int R, int T, bool cur, int n)
+{
+    const size_t base = (tile_smem_bytes(nl, R, T, true, cur, false) + 15) / 16 * 16;
+    return base + 4 * ((size_t)n + (n + 31) / 32 + nl + 1);
+}
+
+template <bool CUR>
+__global__ void __launch_bounds__(kTileThreads, 1) k_tile_stdp(StepArgs a, TileArgs t, int32_t nsteps)
+{
+    extern __shared__ __align__(16) unsigned char tile_raw[];
+    __shared__ int abort_flag;
+    __shared__ unsigned long long blk_ev;
+    __shared__ int count, npg, total;
+    __shared__ uint32_t mine[kTileInline];
+    __shared__ int scnt[kTileWindow];
+    __shared__ int32_t sbase[2], stot;   // places reserved in a step, a step's spikes
+    const TileSmem m = tile_smem<CUR, true>(tile_raw, t);
+    TileStdpSmem q;
+    {
+        unsigned char* p = tile_raw + (tile_smem_bytes(t.nl, t.R, t.T, true, CUR, false) + 15) / 16 * 16;
+        q.lf = reinterpret_cast<int32_t*>(p);
+        q.fired = reinterpret_cast<uint32_t*>(q.lf + a.n);
+        q.in_off = q.fired + (a.n + 31) / 32;
+    }
+    const int tile = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    const int64_t s0 = *a.step;
+    const int32_t slot0 = a.slots[0];
+    const bool rec_on = a.record != 0;
+    int64_t rbase = rec_on ? *a.raster_pos : 0;
+    const int64_t rstep0 = *a.raster_step0;
+    const int64_t s_end = s0 + nsteps;
+    unsigned long long ev = 0;
+    uint2* rec = reinterpret_cast<uint2*>(const_cast<void*>(t.rec));
+    unsigned long long* ring = reinterpret_cast<unsigned long long*>(m.ring);
+    const int plane = t.R * t.stride;
+    unsigned long long* gring[2] = {reinterpret_cast<unsigned long long*>(a.ring_e),
+                                    reinterpret_cast<unsigned long long*>(a.ring_i)};
+
+    // state of the tile, the pending input of steps s0 .. s0 + R - 1
+    for (int i = tid; i < t.nl; i += blockDim.x) {
+        const int32_t gi = tile_neuron(t, i, tile);
+        const bool in = gi < a.ns;
+        m.type[i] = in ? a.type[gi] : (int8_t)kRAW;
+        m.V[i] = in ? a.V[gi] : 0.f;
+        m.rf[i] = in ? a.refrac[gi] : 0;
+        if (CUR) {
+            m.ie[i] = in ? a.Iexc[gi] : 0.f;
+            m.ii[i] = in ? a.Iinh[gi] : 0.f;
+        }
+        for (int x = 0; x < t.R; ++x) {
+            const int row = (int)((s0 + x) % t.R);
+            const size_t from = (size_t)((slot0 + x) % a.M) * (size_t)a.ns + gi;
+            for (int h = 0; h < 2; ++h) ring[h * plane + row * t.stride + i] = in ? gring[h][from] : 0ull;
+        }
+    }
+    for (int i = tid; i < a.n; i += blockDim.x) q.lf[i] = a.last_fired[i];
+    for (int i = tid; i < (a.n + 31) / 32; i += blockDim.x) q.fired[i] = 0;
+    for (int i = tid; i <= t.nl; i += blockDim.x) q.in_off[i] = t.in_off[(size_t)tile * t.nl + i];
+    if (tid < kTileWindow) scnt[tid] = 0;
+    if (tid == 0) {
+        abort_flag = 0;
+        blk_ev = 0;
+        count = npg = total = 0;
+    }
+    __syncthreads();
+    for (int g = tid; g < t.nl / 4; g += blockDim.x) {
+        bool p = false;
+        for (int x = 0; x < 4; ++x) p |= m.type[4 * g + x] == kPOISSON;
+        if (p) m.pg[atomicAdd(&npg, 1)] = (uint16_t)g;
+    }
+    __syncthreads();
+    const int n_pg = npg;
+    const size_t list_len = (size_t)t.nl * t.W;
+    auto my_list = [&](int k) { return t.list + ((size_t)(k & 1) * t.T + tile) * list_len; };
+    // f(id) for every spike of the step, the block's threads (or groups of
+    // `width` of them) in turn
+    auto each_spike = [&](int k, int group, int groups, auto f) {
+        if (total <= kTileSpikes) {
+            for (int x = group; x < total; x += groups) f((int32_t)(m.spikes[x] & kTileId));
+        } else {
+            const uint32_t* lists = t.list + (size_t)(k & 1) * t.T * list_len;
+            for (int l = 0; l < t.T; ++l)
+                for (int x = group; x < m.cnt[l]; x += groups) f((int32_t)(__ldcg(lists + (size_t)l * list_len + x) & kTileId));
+        }
+    };
+    // raster places of step x's spikes (the step's counter is final), one step late
+    auto record = [&](int k, int64_t x, int c) {
+        for (int y = tid; y < c; y += blockDim.x) {
+            const int32_t id = (int32_t)(my_list(k)[y] & kTileId);
+            const int64_t rb = rbase + atomicAdd(&sbase[k & 1], 1);  // any order inside a step
+            if (rec_on && rb < a.raster_ids_cap) a.raster_ids[rb] = id;
+            ev += (unsigned long long)(a.row_ptr[id + 1] - a.row_ptr[id]);
+        }
+        if (tile == 0 && tid == 0 && rec_on) {
+            if (x - rstep0 < a.raster_steps_cap)
+                a.raster_counts[x - rstep0] = stot;
+            else
+                atomicOr(a.status, kStatusRasterSteps);
+            if (rbase + stot > a.raster_ids_cap) atomicOr(a.status, kStatusRasterIds);
+        }
+        rbase += stot;
+    };
+    int slot = (int)(s0 % t.R);
+    int k = 0, c_prev = 0;
+    for (int64_t s = s0; s < s_end; ++s, ++k) {
+        if (n_pg) tile_poisson(a, t, m, s, 1, n_pg, my_list(k), mine, &count, scnt);
+        tile_update<CUR, true>(a, t, m, s, 1, slot, false, my_list(k), mine, &count, scnt);
+        if (tile == 0 && tid == 0) t.cnt[((k + 1) & 3) * kTileWindow] = 0;
+        __syncthreads();
+        const int c_now = count;
+        tile_publish(t, k, c_now, mine, tile == 0);  // (tile 0 cleared a counter)
+        int place = 0;
+        if (tid == 32 && c_now) place = atomicAdd(t.cnt + (k & 3) * kTileWindow, c_now);
+        if (!tile_gather(a, t, m, k, t.list + (size_t)(k & 1) * t.T * list_len, list_len, &total, &abort_flag)) return;
+        if (tid == 32) {
+            sbase[k & 1] = place;
+            scnt[0] = 0;
+        }
+        if (tid == 0) {
+            count = 0;
+            if (k > 0) stot = __ldcg(t.cnt + ((k - 1) & 3) * kTileWindow);
+        }
+        each_spike(k, tid, blockDim.x, [&](int32_t id) {
+            if (!MGC_OK_INDEX(id >= 0 && id < a.n)) return;
+            q.lf[id] = (int32_t)s;
+            atomicOr(q.fired + (id >> 5), 1u << (id & 31));
+        });
+        __syncthreads();
+        // this tile's synapses of the spiking sources, eight lanes a source
+        each_spike(k, tid >> 3, blockDim.x >> 3, [&](int32_t id) {
+            if (!MGC_OK_INDEX(id >= 0 && id < a.n)) return;
+            const uint32_t* o = t.off + (size_t)id * t.T + tile;
+            const uint32_t b = __ldg(o), e = __ldg(o + 1);
+            if (!MGC_OK_INDEX(b <= e && e <= t.n_vec)) return;
+            for (uint32_t r0 = b + (lane & 7); r0 < e; r0 += 32) {
+                uint2 x[4];
+                uint32_t cp[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (r0 + 8 * u < e) {
+                        x[u] = __ldcg(rec + r0 + 8 * u);
+                        cp[u] = __ldg(t.cpos + r0 + 8 * u);
+                    }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    if (r0 + 8 * u >= e) continue;
+                    const int local = (int)(x[u].x & 0xffffu), d = (int)((x[u].x >> 16) & 0x7fffu);
+                    int row = slot + d;
+                    if (row >= t.R) row -= t.R;
+                    if (!MGC_OK_INDEX(local < t.nl && row < t.R && cp[u] < (uint64_t)a.n_syn)) continue;
+                    const float w = as_f(x[u].y);
+                    atomicAdd(ring + (w > 0.0f ? 0 : plane) + row * t.stride + local,
+                              (unsigned long long)to_fx(w, a.fx_scale));
+                    if (x[u].x >> 31) {
+                        const uint32_t nw = as_u(stdp_weight((int32_t)s - q.lf[tile_neuron(t, local, tile)], w, a.P));
+                        rec[r0 + 8 * u].y = nw;
+                        a.syn[cp[u]].y = nw;
+                    }
+                }
+            }
+        });
+        // the plastic synapses onto this tile's spiking neurons, the block on each
+        for (int y = 0; y < c_now; ++y) {
+            const int32_t id = (int32_t)((y < kTileInline ? mine[y] : __ldcg(my_list(k) + y)) & kTileId);
+            const int g = id >> 2, local = g / t.T * 4 + (id & 3);
+            const uint32_t e = q.in_off[local + 1];
+            for (uint32_t p0 = q.in_off[local] + tid; p0 < e; p0 += 2 * blockDim.x) {
+                uint2 en[2];
+                uint32_t w[2], cp[2];
+                bool go[2];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    go[u] = p0 + u * blockDim.x < e;
+                    if (go[u]) en[u] = __ldg(t.in_ent + p0 + u * blockDim.x);
+                }
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    go[u] = go[u] && MGC_OK_INDEX(en[u].x < (uint32_t)a.n && en[u].y < t.n_vec) &&
+                            !bit_of(q.fired, (int32_t)en[u].x);
+                    if (go[u]) {
+                        w[u] = __ldcg(&rec[en[u].y].y);
+                        cp[u] = __ldg(t.cpos + en[u].y);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    if (!go[u]) continue;
+                    const uint32_t nw = as_u(stdp_weight(q.lf[en[u].x] - (int32_t)s, as_f(w[u]), a.P));
+                    rec[en[u].y].y = nw;
+                    a.syn[cp[u]].y = nw;
+                }
+            }
+        }
+        __syncthreads();
+        each_spike(k, tid, blockDim.x, [&](int32_t id) { q.fired[id >> 5] = 0; });
+        if (k > 0) record(k - 1, s - 1, c_prev);
+        c_prev = c_now;
+        slot = slot + 1 == t.R ? 0 : slot + 1;
+        __syncthreads();
+        if (tid == 0) total = 0;
+    }
+    // the last step's raster: an empty window makes its counter final
+    __syncthreads();
+    tile_publish(t, k, 0, mine, true);
+    if (!tile_gather(a, t, m, k, t.list, 0, &total, &abort_flag)) return;
+    if (tid == 0) stot = __ldcg(t.cnt + ((k - 1) & 3) * kTileWindow);
+    __syncthreads();
+    record(k - 1, s_end - 1, c_prev);
+    for (int i = tid; i < t.nl; i += blockDim.x) {
+        const int32_t gi = tile_neuron(t, i, tile);
+        if (gi >= a.ns) continue;
+        const int32_t slot_end = (int32_t)((slot0 + nsteps) % a.M);
+        const bool pois = m.type[i] == kPOISSON;
+        for (int x = 0; x < a.M; ++x) {
+            const int row = (int)((s_end + x) % t.R);
+            const size_t to = (size_t)((slot_end + x) % a.M) * (size_t)a.ns + gi;
+            for (int h = 0; h < 2; ++h)  // (a POISSON neuron's input is read by nobody)
+                gring[h][to] = x < t.R && !pois ? ring[h * plane + row * t.stride + i] : 0ull;
+        }
+        if (pois) continue;
+        a.V[gi] = m.V[i];
+        a.refrac[gi] = m.rf[i];
+        if (CUR) {
+            a.Iexc[gi] = m.ie[i];
+            a.Iinh[gi] = m.ii[i];
+        }
+    }
+    if (ev) atomicAdd(&blk_ev, ev);
+    __syncthreads();
+    if (tid == 0 && blk_ev) atomicAdd(a.events, blk_ev);
+    if (last_block(a.done) && tid == 0) {
+        if (rec_on) *a.raster_pos = rbase;
+        for (int j = 0; j < 4 * kTileWindow; ++j) t.cnt[j] = 0;
+        *a.done = 0;
+        a.slots[0] = (int32_t)((slot0 + nsteps) % a.M);
         *a.step = s_end;
     }
 }

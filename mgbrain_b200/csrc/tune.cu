@@ -16,6 +16,7 @@ mgc_status mgc_profile_steps(mgc_sim* s, int64_t steps, float* ms)
     std::vector<cudaEvent_t> ev(4 * kBatch);
     for (auto& e : ev) CK(cudaEventCreate(&e));
     double acc[3] = {0, 0, 0};
+    if (s->stdp && s->tile_ok && steps > 0) s->tile_stale = true;
     // External records become event-record nodes of the captured graph (a
     // plain record inside a capture only orders the capture's streams).
     auto rec = [&](cudaEvent_t ev_) { cudaEventRecordWithFlags(ev_, s->stream, cudaEventRecordExternal); };
@@ -350,7 +351,7 @@ mgc_status mgc_autotune(mgc_sim* s, int64_t steps_per_trial, mgc_tune_report* re
     // the tiled step group, where the network has its layout: it runs in the
     // place of the builder's default step-group mode
     if (s->tile_ok && st == MGC_OK && !sched_wanted(s)) {
-        s->persistent = s->dmin >= 4 ? 2 : 1;
+        s->persistent = !s->a.deferred ? 0 : (s->dmin >= 4 ? 2 : 1);
         s->tile_on = true;
         st = mgc_run(s, kGraphSteps);
         if (st == MGC_OK) {
