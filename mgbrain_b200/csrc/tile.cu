@@ -6,7 +6,6 @@ namespace mgc {
 namespace {
 
 constexpr int kTileRowBlock = 256;
-constexpr int kMaxTiles = 256;
 // Above this many neurons, networks with fewer than 4 records a segment keep the
 // other step groups: every tile looks up a segment per spike, and at 200,000
 // neurons with 2 records a segment a driven step took 9.3 us against 5.8 for
@@ -255,7 +254,7 @@ mgc_status build_tiles(mgc_sim* s)
     // at most one vector in each segment is not full
     const size_t most = ((size_t)s->S / 2 + (size_t)s->n * T) * vec_bytes;
     const int W = stdp ? 1 : std::min(kTileWindow, s->dmin);
-    const size_t need = most + (stdp ? 12 * (size_t)s->S : 0) + ((size_t)s->n * T + 1) * 4 + 2 * (size_t)W * nl_of(T) * T * 4 + 16 * (size_t)a.ns;
+    const size_t need = most + (stdp ? 12 * (size_t)s->S : 0) + ((size_t)s->n * T + 1) * 4 + 2 * (size_t)W * nl_of(T) * T * 4 + 32 * (size_t)T * T * kTileChunks + 16 * (size_t)a.ns;
     // offsets in vectors, and in records while they are filled
     if ((int64_t)s->n * T + 1 > (int64_t)0x7fffffff || most / vec_bytes > kIndex / 2) return MGC_OK;
     size_t free_b = 0, total_b = 0;
@@ -275,9 +274,9 @@ mgc_status build_tiles(mgc_sim* s)
     CKS(s->alloc(&off, (size_t)s->n * T + 1, false));
     t.off = off;
     CKS(s->alloc(&t.list, 2 * (size_t)T * t.nl * W, false));
-    CKS(s->alloc(&t.mail, 2 * (size_t)T * T));
+    CKS(s->alloc(&t.mail, 2 * (size_t)T * T * kTileChunks));
     t.epoch = 1;
-    CKS(s->alloc(&t.cnt, 4 * kTileWindow));
+    CKS(s->alloc(&t.cnt, 4 * kTileWindow * kTileLine));
     DevTmp t_deg, t_stat;
     uint32_t *indeg = nullptr, *wstat = nullptr;
     if (!fx) {

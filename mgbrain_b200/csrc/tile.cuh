@@ -42,16 +42,17 @@
 // start a step without its arrivals; there the prologue includes them and
 // the accumulators stay empty.
 //
-// Exchange of window k: a tile writes its spikes (id, step in the window) into
-// its list of buffer k & 1, then sends every tile a 16-byte header {epoch of
-// the window and count, first two spikes}, one store each, into that tile's
-// mailbox; thread l of a block polls the place of tile l in its own mailbox,
-// which no other block reads.  No counter is shared, so no atomic waits its
-// turn, no line is polled by more than one block, and a quiet window's spikes
-// arrive with the poll; only a tile with more spikes than the header carries
-// orders its list before the header with a fence, and only their readers
-// wait for one.  (One set of headers polled by all blocks, with a release
-// store: 5.0 us an exchange on 148 tiles; mailboxes: see DESIGN.)  A tile
+// Exchange of window k: a tile sends every tile its spikes (id, step in the
+// window) in 16-byte chunks, one store each, into that tile's mailbox: {epoch of
+// the window and count, first two spikes}, then {epoch, three spikes}.  Every
+// chunk carries the epoch, so none has to be ordered after another, and no
+// fence is needed; thread l of a block polls the place of tile l in its own
+// mailbox, which no other block reads, so no counter or line is shared.  Only a
+// tile with more spikes than a mailbox holds sends just the count and writes
+// them to its list of buffer k & 1, with a fence before and at its readers.
+// (11,000 neurons: 5.0 us an exchange with one set of headers polled by all
+// blocks and release stores, 2.1 with mailboxes; 44,700 neurons, 13 spikes a
+// tile and window: 8.0 us with two spikes a header and fenced lists.)  A tile
 // overwrites a buffer two windows later, when every tile has published the
 // window between, which it does after reading the buffer.  Waits are bounded
 // (kStatusBarrier).
@@ -59,10 +60,17 @@
 // Raster: a step's place in it needs the step's spikes of all tiles, so each
 // tile adds its counts to the window's 16 step counters when it publishes,
 // and writes its spikes' places one window later, when every tile's counts
-// are in: none of it is waited for.  The counters of window k (slot k % 4)
-// are read in window k+1 before its deliveries end and cleared by tile 0 in
-// window k+3, before anyone adds to them again in window k+4.
+// are in: none of it is waited for.  The counters (slot k % 4) run on over the
+// windows of a launch; every block keeps their last totals.
+//
+// Measured per step, the faster of the other step groups and this one: 4,000
+// neurons, minimum delay 1: 6.5 and 3.2 us; 11,000 neurons, windows of 15 steps
+// quiet: 5.0 and 0.31, with volleys: 8.7 and 1.35; balanced networks of 1e8
+// synapses, quiet: 6.6 and 0.98, and of 3e7 at POISSON rates of 1 kHz: 20.9 and
+// 4.7; 9,000 neurons with a range of delays: 7.8 and 1.1.
 #pragma once
+#include <type_traits>
+
 #include "kernels.cuh"
 
 namespace mgc {
@@ -75,7 +83,7 @@ constexpr int kTileTable = 512;     // entries of each chain table
 struct TileArgs {
     int32_t T;            // tiles = blocks
     int32_t nl;           // neurons per tile (a multiple of 4)
-    int32_t stride;       // entries of a ring row: nl, a spare one for fillers, padding
+    int32_t stride;       // entries of a ring row: nl, one for fillers, an empty one, padding
     int32_t R;            // ring slots: the longest delay
     int32_t W;            // steps per window (<= minimum delay)
     int32_t dmin, dmax;
@@ -89,17 +97,21 @@ struct TileArgs {
     const float* wi;
     const float* chain;   // [2][kTileTable] sums of k weights (exc, inh), when table
     uint32_t* list;       // [2][T][nl*W] spikes of a window: id | step in the window << 28
-    ulonglong2* mail;     // [2][T reader][T] headers {epoch << 32 | count, first spikes}
+    ulonglong2* mail;     // [2][T reader][T][kTileChunks]
     uint32_t epoch;       // epoch of the launch's first window (they count on over the launches)
-    int32_t* cnt;         // [4][kTileWindow] spikes of a window's steps; zero between launches
+    int32_t* cnt;         // [4][kTileWindow] counters (tile_counter) of a window's steps' spikes; zero between launches
     // plastic networks (k_tile_stdp): rec holds single records (off counts them)
     const uint32_t* cpos;   // [S] CSR position of a record
     const uint32_t* in_off; // [T*nl + 1] plastic synapses onto each local neuron, tile after tile:
     const uint2* in_ent;    //   {source, record}
 };
 
-constexpr int kTileInline = 2;      // spikes a header carries
-constexpr int kTileSpikes = 4096;   // spikes of a window gathered in shared memory
+constexpr int kTileLine = 32;       // a counter has a line to itself: 148 blocks add to 16 of them at once, and
+                                    // on one line those atomics queued for 8 to 70 us a window
+constexpr int kTileChunks = 16;     // chunks of a mailbox place
+constexpr int kTileInline = 2 + 3 * (kTileChunks - 1);  // spikes they carry
+constexpr int kTileSpikes = 8192;   // spikes of a window gathered in shared memory; every mailbox full fits
+constexpr int kMaxTiles = kTileSpikes / kTileInline;
 constexpr int kTileStepShift = 28;  // spike word: id below, step in the window above
 
 // Shared memory of a block, in this order.
@@ -114,7 +126,7 @@ struct TileSmem {
     int8_t* type;
 };
 
-// A ring row: nl entries and the fillers' one, a multiple of 4.
+// A ring row: nl entries, the fillers' one and an empty one, a multiple of 4.
 __host__ __device__ inline int tile_stride(int nl) { return nl + 4; }
 
 __host__ __device__ inline int tile_lists(int R, int T) { return R > T ? R : T; }
@@ -159,6 +171,11 @@ __device__ __forceinline__ TileSmem tile_smem(unsigned char* base, const TileArg
     return m;
 }
 
+__device__ __forceinline__ int32_t* tile_counter(const TileArgs& t, int k, int j)
+{
+    return t.cnt + ((k & 3) * kTileWindow + j) * kTileLine;
+}
+
 // Network neuron of local neuron i of this block's tile.
 __device__ __forceinline__ int32_t tile_neuron(const TileArgs& t, int i, int tile)
 {
@@ -174,6 +191,7 @@ __device__ __forceinline__ float chain_sum(uint32_t c, float w, const float* tab
         v = tab[k];
         c -= k;
     }
+#pragma unroll 1
     for (; c; --c) v = fadd_ftz(v, w);
     return v;
 }
@@ -183,6 +201,7 @@ __device__ __forceinline__ void tile_spikes(const TileArgs& t, int32_t gi, uint3
                                             uint32_t* first, int* count, int* scnt)
 {
     int pos = atomicAdd(count, __popc(fm));
+#pragma unroll 1
     for (; fm; fm &= fm - 1, ++pos) {
         const int j = __ffs(fm) - 1;
         atomicAdd(scnt + j, 1);
@@ -198,28 +217,117 @@ __device__ __forceinline__ void tile_spikes(const TileArgs& t, int32_t gi, uint3
 __device__ __forceinline__ void tile_poisson(const StepArgs& a, const TileArgs& t, const TileSmem& m, int64_t w0,
                                              int wl, int npg, uint32_t* list, uint32_t* first, int* count, int* scnt)
 {
+#pragma unroll 1
     for (int x = blockDim.x - 1 - threadIdx.x; x < npg * wl; x += blockDim.x) {
         const int j = x / npg, g = m.pg[x - j * npg];
         const int32_t gi = tile_neuron(t, 4 * g, blockIdx.x);
-        float u[4];
-        poisson_uniform4(a.seed, (int64_t)gi + a.id_offset, w0 + j, u);
+        const int64_t id = (int64_t)gi + a.id_offset;
+        float u[4] = {0.f, 0.f, 0.f, 0.f};
+        if ((id & 3) == 0) {
+            const uint64_t st = (uint64_t)(w0 + j);
+            const U32x4 r = philox4x32_10((uint32_t)st, (uint32_t)(st >> 32), (uint32_t)((uint64_t)id >> 2),
+                                          kTagPoisson, (uint32_t)a.seed, (uint32_t)(a.seed >> 32));
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            if (m.type[4 * g + q] != kPOISSON || !(m.V[4 * g + q] > u[q])) continue;  // (V holds the probability)
-            atomicAdd(a.fire_cnt + gi + q, 1);
-            atomicMax(a.last_fired + gi + q, (int32_t)(w0 + j));  // another thread has the group's other steps
-            tile_spikes(t, gi + q, 1u << j, list, first, count, scnt);
+            for (int q = 0; q < 4; ++q) u[q] = unit_open0(pick(r, q));
+        } else {  // ids that start inside a Philox block
+#pragma unroll 1
+            for (int q = 0; q < 4; ++q) {
+                const float x = poisson_uniform(a.seed, id + q, w0 + j);
+#pragma unroll
+                for (int y = 0; y < 4; ++y) u[y] = y == q ? x : u[y];
+            }
+        }
+        unsigned f = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q)  // (V holds the probability)
+            f |= (m.type[4 * g + q] == kPOISSON && m.V[4 * g + q] > u[q] ? 1u : 0u) << q;
+#pragma unroll 1
+        for (; f; f &= f - 1) {
+            const int32_t nrn = gi + __ffs(f) - 1;
+            atomicAdd(a.fire_cnt + nrn, 1);
+            atomicMax(a.last_fired + nrn, (int32_t)(w0 + j));  // another thread has the group's other steps
+            tile_spikes(t, nrn, 1u << j, list, first, count, scnt);
+        }
+    }
+}
+
+// Inputs of the steps whose ring words are at[0..N), which are cleared.
+template <bool FX, int N>
+__device__ __forceinline__ void tile_inputs(const StepArgs& a, const TileArgs& t, const TileSmem& m, const int* at,
+                                            float we, float wi, float* re, float* ri)
+{
+    if (FX) {
+        const int plane = t.R * t.stride;  // the inh sums follow the exc ones
+        long long* ring = reinterpret_cast<long long*>(m.ring);
+        long long fe[N], fi[N];
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            fe[k] = ring[at[k]];
+            fi[k] = ring[plane + at[k]];
+            ring[at[k]] = 0;
+            ring[plane + at[k]] = 0;
+        }
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            re[k] = from_fx(fe[k], a.fx_unscale);
+            ri[k] = from_fx(fi[k], a.fx_unscale);
+        }
+        return;
+    }
+    uint32_t* ring = reinterpret_cast<uint32_t*>(m.ring);
+    constexpr uint32_t kMask = kTileTable - 1;
+    uint32_t c[N], any = 0;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        c[k] = ring[at[k]];
+        ring[at[k]] = 0;
+        any |= c[k];
+    }
+    if (m.tab && !__any_sync(0xffffffffu, (any & ~(kMask | (kMask << 16))) != 0)) {  // (tab[0] is 0)
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            re[k] = m.tab[c[k] & kMask];
+            ri[k] = m.tab[kTileTable + (c[k] >> 16)];
+        }
+        return;
+    }
+    // counts past the tables, or no tables: all chains an addition at a time
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        re[k] = ri[k] = 0.0f;
+        if (m.tab) {
+            const uint32_t ce = min(c[k] & 0xffffu, kMask), ci = min(c[k] >> 16, kMask);
+            re[k] = m.tab[ce];
+            ri[k] = m.tab[kTileTable + ci];
+            c[k] -= ce | (ci << 16);
+        }
+    }
+#pragma unroll 1
+    while (__any_sync(0xffffffffu, any != 0)) {
+        any = 0;
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            if (c[k] & 0xffffu) {
+                re[k] = fadd_ftz(re[k], we);
+                c[k] -= 1u;
+            }
+            if (c[k] >> 16) {
+                ri[k] = fadd_ftz(ri[k], wi);
+                c[k] -= 0x10000u;
+            }
+            any |= c[k];
         }
     }
 }
 
 // The tile's other neurons through the wl steps from w0 (ring slot `slot`),
-// one neuron a lane, four steps at a time.  `from_acc`: the first step's
+// one neuron a lane, eight steps at a time.  `from_acc`: the first step's
 // input is in the accumulators (the launch's first step), which are cleared.
 // The spikes go into `list` (and `first`), counted in *count and per step.
-// Warps without LIF or LIFE neurons take lifb_step for every lane and keep
-// its result where the neuron is LIFB: no branches, few instructions (a
-// window's update is one warp's chain of dependent instructions).
+// Warps without LIF or LIFE neurons take lifb_step for every lane, whatever its
+// neuron, and keep the result of LIFB neurons at the end; lanes without input,
+// and steps past the window, read a column of the rows that stays empty, so
+// that a batch has no branches.
 template <bool CUR, bool FX>
 __device__ __forceinline__ void tile_update(const StepArgs& a, const TileArgs& t, const TileSmem& m, int64_t w0,
                                             int wl, int slot, bool from_acc, uint32_t* list, uint32_t* first,
@@ -227,7 +335,7 @@ __device__ __forceinline__ void tile_update(const StepArgs& a, const TileArgs& t
 {
     const int lane = threadIdx.x & 31;
     const int tile = blockIdx.x;
-    const int plane = t.R * t.stride;  // fixed point: the inh sums follow the exc ones
+#pragma unroll 1
     for (int b = threadIdx.x - lane; b < t.nl; b += blockDim.x) {
         const int i = b + lane;
         const int type = i < t.nl ? m.type[i] : (int)kRAW;
@@ -248,69 +356,21 @@ __device__ __forceinline__ void tile_update(const StepArgs& a, const TileArgs& t
                 ii = m.ii[i];
             }
         }
-        const bool lifb = type == kLIFB;
         const bool any_cur = CUR && __any_sync(0xffffffffu, type == kLIF || type == kLIFE);
         uint32_t fm = 0;
-        int row = slot;
-#pragma unroll 1
-        for (int h = 0; h < wl; h += 4) {
-            float re[4], ri[4];
-            int at[4];
+        const int empty = t.nl + 1, wrap = t.R * t.stride;
+        int place = slot * t.stride + (input ? i : empty);
+        auto batch = [&](auto width, int h, int n) {
+            constexpr int N = decltype(width)::value;
+            float re[N], ri[N];
+            int at[N];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                at[k] = row * t.stride + i;
-                row = row + 1 == t.R ? 0 : row + 1;
+            for (int k = 0; k < N; ++k) {
+                at[k] = N == 1 || k < n ? place : empty;
+                place += t.stride;
+                place = place >= wrap ? place - wrap : place;
             }
-            if (FX) {
-                long long* ring = reinterpret_cast<long long*>(m.ring);
-                long long fe[4], fi[4];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    fe[k] = fi[k] = 0;
-                    if (input && h + k < wl) {
-                        fe[k] = ring[at[k]];
-                        fi[k] = ring[plane + at[k]];
-                    }
-                }
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    if (fe[k] | fi[k]) ring[at[k]] = ring[plane + at[k]] = 0;
-                    re[k] = from_fx(fe[k], a.fx_unscale);
-                    ri[k] = from_fx(fi[k], a.fx_unscale);
-                }
-            } else {
-                uint32_t* ring = reinterpret_cast<uint32_t*>(m.ring);
-                uint32_t c[4];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    c[k] = 0;
-                    if (input && h + k < wl) {
-                        c[k] = ring[at[k]];
-                        ring[at[k]] = 0;
-                    }
-                }
-                if (m.tab) {  // tab[0] is 0; counts past the tables are finished one by one
-                    constexpr uint32_t kMask = kTileTable - 1;
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        re[k] = m.tab[c[k] & kMask];
-                        ri[k] = m.tab[kTileTable + ((c[k] >> 16) & kMask)];
-                    }
-                    if ((c[0] | c[1] | c[2] | c[3]) & ~(kMask | (kMask << 16))) {
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            re[k] = chain_sum(c[k] & 0xffffu, we, m.tab);
-                            ri[k] = chain_sum(c[k] >> 16, wi, m.tab + kTileTable);
-                        }
-                    }
-                } else {
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        re[k] = chain_sum(c[k] & 0xffffu, we, nullptr);
-                        ri[k] = chain_sum(c[k] >> 16, wi, nullptr);
-                    }
-                }
-            }
+            tile_inputs<FX, N>(a, t, m, at, we, wi, re, ri);
             if (from_acc && h == 0 && input && gi < a.ns) {
                 typename AccT<FX>::type* pe = acc_buf<FX>(a, a.acc_e, w0) + gi;
                 typename AccT<FX>::type* pi = acc_buf<FX>(a, a.acc_i, w0) + gi;
@@ -324,37 +384,38 @@ __device__ __forceinline__ void tile_update(const StepArgs& a, const TileArgs& t
                 *pe = 0;
                 *pi = 0;
             }
-            if (any_cur) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    if (h + k < wl && input)
-                        fm |= (update_one<false>(a, type, gi, w0 + h + k, v, rf, re[k], ri[k], ie, ii, 0.f) ? 1u : 0u)
-                              << (h + k);
-            } else {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    float nv = v;
-                    int32_t nr = rf;
-                    const bool go = lifb && h + k < wl;  // the window's last batch may be partial
-                    const bool f = lifb_step(a, nv, nr, re[k], ri[k]) && go;
-                    v = go ? nv : v;
-                    rf = go ? nr : rf;
-                    fm |= (f ? 1u : 0u) << (h + k);
-                }
+            for (int k = 0; k < N; ++k) {
+                if (N > 1 && k >= n) break;
+                bool f;
+                if (any_cur)
+                    f = input && update_one<false>(a, type, gi, w0 + h + k, v, rf, re[k], ri[k], ie, ii, 0.f);
+                else
+                    f = lifb_step(a, v, rf, re[k], ri[k]);
+                fm |= (f ? 1u : 0u) << (h + k);
             }
+        };
+        constexpr int kWide = CUR ? 4 : 8;  // (update_one is long: fewer copies of it)
+        int h = 0;
+#pragma unroll 1
+        for (; wl - h > 1; h += kWide) {
+            if (!CUR && wl - h <= 4)
+                batch(std::integral_constant<int, 4>{}, h, wl - h);
+            else
+                batch(std::integral_constant<int, kWide>{}, h, wl - h);
         }
-        if (input) {
-            m.V[i] = v;
-            m.rf[i] = rf;
-            if (CUR) {
-                m.ie[i] = ie;
-                m.ii[i] = ii;
-            }
-            if (fm) {
-                atomicAdd(a.fire_cnt + gi, __popc(fm));
-                a.last_fired[gi] = (int32_t)(w0 + (31 - __clz(fm)));
-                tile_spikes(t, gi, fm, list, first, count, scnt);
-            }
+        if (wl - h == 1) batch(std::integral_constant<int, 1>{}, h, 1);
+        if (!input || !(any_cur || type == kLIFB)) continue;
+        m.V[i] = v;
+        m.rf[i] = rf;
+        if (CUR) {
+            m.ie[i] = ie;
+            m.ii[i] = ii;
+        }
+        if (fm) {
+            atomicAdd(a.fire_cnt + gi, __popc(fm));
+            a.last_fired[gi] = (int32_t)(w0 + (31 - __clz(fm)));
+            tile_spikes(t, gi, fm, list, first, count, scnt);
         }
     }
 }
@@ -412,65 +473,99 @@ __device__ __forceinline__ void tile_apply_vec(const StepArgs& a, const TileArgs
     }
 }
 
-// Where a warp's batches of spikes come from: begin(n) starts its next batch
-// (false: none left; n <= 32 U spikes), load(i, j) returns spike i of the batch
-// and its step (j steps after the first).
-constexpr int kTileU = 2;           // segments a lane takes in a batch
+// 2, 3 and 4 segments (2, 6 and 8 vectors) a lane ran no faster on driven
+// networks, and their code is longer, which every quiet window pays for.
+constexpr int kTileU = 1;           // segments a lane takes in a batch
 constexpr int kTileD = 4;           // 8-byte vectors of each it loads at once (half as many of 16)
 constexpr int kTileBatch = 32 * kTileU;
 constexpr uint32_t kTileId = (1u << kTileStepShift) - 1u;
 
-struct TileGathered {  // the window's spikes in shared memory
-    const uint32_t* spikes;
-    int total, per, next, at;
-    __device__ TileGathered(const uint32_t* sp, int n) : spikes(sp), total(n)
+// Tile l's list in window k, and spike q of the tile from its mailbox place.
+__device__ __forceinline__ const uint32_t* tile_list(const TileArgs& t, int k, int l)
+{
+    return t.list + ((size_t)(k & 1) * t.T + l) * ((size_t)t.nl * t.W);
+}
+__device__ __forceinline__ uint32_t tile_mail(const TileArgs& t, int k, int l, int q)
+{
+    const uint32_t* p = reinterpret_cast<const uint32_t*>(
+        t.mail + (((size_t)(k & 1) * t.T + blockIdx.x) * t.T + l) * kTileChunks);
+    const int g = q < 2 ? 0 : (q - 2) / 3 + 1;  // words: count, epoch, 2 spikes; then spike, epoch, 2 spikes
+    const int r = q < 2 ? q + 2 : q - 2 - 3 * (g - 1);
+    return __ldcg(p + 4 * g + (q < 2 ? r : (r == 0 ? 0 : r + 1)));
+}
+
+// Where a warp's batches of spikes come from: the window's spikes gathered in
+// shared memory, the tiles' mailboxes and lists of a window with more, or the
+// history's lists (the prologue); lists are cut into batches dealt to the
+// block's warps in turn.  One struct for the three, so that the delivery is
+// in the code once (the kernel's loop is run through once a window, and
+// instruction fetches are a good part of a quiet window).
+struct TileSource {
+    enum { kGathered, kTiles, kHistory };
+    int kind, k;              // k: the window
+    int total, per, next;     // gathered
+    int lists, l, q, skip;    // lists: m.cnt holds their lengths
+    int at;                   // the batch's first spike
+    const uint32_t* from;     // its list (null: the mailbox)
+    int32_t h0;               // history slot of the first list
+
+    __device__ __forceinline__ void gathered(int n)
     {
+        kind = kGathered;
+        total = n;
         const int nw = blockDim.x >> 5, need = (n + nw - 1) / nw;
         per = need < kTileBatch ? (need > 0 ? need : 1) : kTileBatch;
         next = (threadIdx.x >> 5) * per;
-        at = 0;
     }
-    __device__ __forceinline__ bool begin(int& n)
+    __device__ __forceinline__ void listed(int kind_, int n, int k_or_slot)
     {
-        at = next;
-        n = min(per, total - at);
-        next += (blockDim.x >> 5) * per;
-        return n > 0;
-    }
-    __device__ __forceinline__ int32_t load(int i, int& j) const
-    {
-        const uint32_t e = spikes[at + i];
-        j = (int)(e >> kTileStepShift);
-        return (int32_t)(e & kTileId);
-    }
-};
-
-// Lists in device memory (get(l, q, j): spike q of list l), cut into batches
-// dealt to the block's warps in turn; cnt: their lengths, in shared memory.
-template <class Get> struct TileListed {
-    Get get;
-    const int32_t* cnt;
-    int lists, l, q, skip, cl, cq;
-    __device__ TileListed(Get g, const int32_t* c, int n) : get(g), cnt(c), lists(n), l(0), q(0), cl(0), cq(0)
-    {
+        kind = kind_;
+        k = h0 = k_or_slot;
+        lists = n;
+        l = q = 0;
         skip = threadIdx.x >> 5;
     }
-    __device__ __forceinline__ bool begin(int& n)
+    // begins the warp's next batch of n <= kTileBatch spikes; false: none left
+    __device__ __forceinline__ bool begin(const StepArgs& a, const TileArgs& t, const TileSmem& m, int& n)
     {
+        if (kind == kGathered) {
+            at = next;
+            n = min(per, total - at);
+            next += (blockDim.x >> 5) * per;
+            return n > 0;
+        }
         q += skip;
         skip = blockDim.x >> 5;
         int b = 0;
+#pragma unroll 1
         for (; l < lists; ++l, q -= b) {
-            b = (cnt[l] + kTileBatch - 1) / kTileBatch;
+            b = (m.cnt[l] + kTileBatch - 1) / kTileBatch;
             if (q < b) break;
         }
         if (l >= lists) return false;
-        cl = l;
-        cq = q * kTileBatch;
-        n = min(kTileBatch, cnt[l] - cq);
+        at = q * kTileBatch;
+        n = min(kTileBatch, m.cnt[l] - at);
+        if (kind == kHistory) {
+            const int h = h0 + l;
+            from = reinterpret_cast<const uint32_t*>(a.hist_ids) + (size_t)(h >= a.H ? h - a.H : h) * (size_t)a.n_src;
+        } else {
+            from = m.cnt[l] > kTileInline ? tile_list(t, k, l) : nullptr;
+        }
         return true;
     }
-    __device__ __forceinline__ int32_t load(int i, int& j) const { return get(cl, cq + i, j); }
+    // spike i of the batch, j steps after the first
+    __device__ __forceinline__ int32_t load(const TileArgs& t, const TileSmem& m, int i, int& j) const
+    {
+        uint32_t e;
+        if (kind == kGathered)
+            e = m.spikes[at + i];
+        else if (from)
+            e = __ldcg(from + at + i);
+        else
+            e = tile_mail(t, k, l, at + i);
+        j = kind == kHistory ? l : (int)(e >> kTileStepShift);
+        return (int32_t)(kind == kHistory ? e : e & kTileId);
+    }
 };
 
 // Delivers spikes of the steps x0, x0+1, ... to this tile's targets: the
@@ -480,144 +575,117 @@ template <class Get> struct TileListed {
 // of this one are in flight together, and a lane loads kTileD vectors of each
 // of its segments at once, so that a batch waits for about one round trip to
 // L2 (walking a segment one vector at a time, with no batch ahead, took 7.6 us
-// a batch).  Long segments are shared by 1 << lanes_log2 lanes.
-template <bool FX, bool ONE, class Src>
+// a batch).  Long segments are cut for 1 << lanes_log2 lanes.
+template <bool FX, bool ONE>
 __device__ __forceinline__ void tile_deliver(const StepArgs& a, const TileArgs& t, const TileSmem& m, int64_t x0,
-                                             int slot0, int64_t lo, int64_t hi, Src src, unsigned long long& events)
+                                             int slot0, int64_t lo, int64_t hi, TileSource src,
+                                             unsigned long long& events)
 {
     using Vec = typename TileVec<FX>::type;
     constexpr int U = kTileU, D = FX ? kTileD / 2 : kTileD;
     const Vec* rec = reinterpret_cast<const Vec*>(t.rec);
     const int lane = threadIdx.x & 31;
+    const int lg = t.lanes_log2;
     // arrival windows relative to x0, as one unsigned comparison
     const int64_t hr = hi - x0, lr = lo - x0;
     const int lo_rel = (int)(lr < -1 ? -1 : lr);
     const int hi_rel = (int)(hr > 4 * kTileMaxDelay ? 4 * kTileMaxDelay : hr);
     const unsigned span = hi_rel > lo_rel ? (unsigned)(hi_rel - lo_rel) : 0u;
     uint32_t ev = 0;
-
-    struct Seg {
-        uint32_t k, e;
-        int base, j;
-    };
-    int32_t id1[U];  // ids and steps of the batch whose offsets come next
+    // a batch of n spikes is n << lg parts of segments; `done` of them taken
+    int n = 0, done = 0;
+    bool more = src.begin(a, t, m, n);
+    int32_t id1[U];   // ids and steps of the parts whose offsets come next
     int j1[U];
-    Seg s0[U];       // segments of the batch to deliver
-    auto ids = [&](bool any, int n) {
+    uint32_t k0[U], e0[U];  // segments of the parts to deliver, their steps
+    int j0[U];
+    auto ids = [&]() {      // the next parts' ids; begins the next batch after the last
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             id1[u] = -1;
             j1[u] = 0;
-            if (any && u * 32 + lane < n) id1[u] = src.load(u * 32 + lane, j1[u]);
+            const int p = done + u * 32 + lane;
+            if (more && (p >> lg) < n) id1[u] = src.load(t, m, p >> lg, j1[u]);
         }
     };
     auto offsets = [&]() {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            Seg& g = s0[u];
-            g.k = g.e = 0;
+            k0[u] = e0[u] = 0;
             if (id1[u] >= 0 && MGC_OK_INDEX(id1[u] < a.n_src)) {
                 const uint32_t* o = t.off + (size_t)id1[u] * t.T + blockIdx.x;
-                g.k = __ldg(o);
-                g.e = __ldg(o + 1);
+                k0[u] = __ldg(o);
+                e0[u] = __ldg(o + 1);
             }
-            g.j = j1[u];
+            j0[u] = j1[u];
         }
     };
-    int n0 = 0, n1 = 0;
-    bool more = src.begin(n1);
+    auto advance = [&]() {  // past the parts whose ids are loaded
+        done += kTileBatch;
+        if (done >= n << lg) {
+            done = 0;
+            more = src.begin(a, t, m, n);
+        }
+    };
     if (!more) return;
-    ids(true, n1);
+    ids();
     offsets();
-    n0 = n1;
-    more = src.begin(n1);
-    ids(more, n1);
-    for (;;) {
-        // this batch's segments, their first vectors
-        Seg c[U];
+    int part = done;  // first part of the batch whose segments come next
+    advance();
+    ids();
+#pragma unroll 1
+    for (bool go = true; go;) {
+        // these parts' segments
+        uint32_t k[U], e[U];
+        int base[U], j[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            c[u] = s0[u];
-            int sl = slot0 + c[u].j;
+            j[u] = j0[u];
+            int sl = slot0 + j[u];
             if (sl >= t.R) sl -= t.R;
+            k[u] = k0[u];
+            e[u] = e0[u];
             if (ONE) {  // (R = dmin: the arrival row is the spike's own)
-                sl = sl * t.stride * 4 + (int)(c[u].k >> 31);
-                c[u].k &= 0x7fffffffu;
-                c[u].e &= 0x7fffffffu;
-                if ((unsigned)(c[u].j + t.dmin - lo_rel - 1) >= span) c[u].e = c[u].k;
+                sl = sl * t.stride * 4 + (int)(k[u] >> 31);
+                k[u] &= 0x7fffffffu;
+                e[u] &= 0x7fffffffu;
+                if ((unsigned)(j[u] + t.dmin - lo_rel - 1) >= span) e[u] = k[u];
             }
-            c[u].base = sl;
-            if (!MGC_OK_INDEX(c[u].k <= c[u].e && c[u].e <= t.n_vec)) c[u].e = c[u].k;
+            base[u] = sl;
+            if (!MGC_OK_INDEX(k[u] <= e[u] && e[u] <= t.n_vec)) e[u] = k[u];
+            if (lg) {
+                const uint32_t len = e[u] - k[u], p = (uint32_t)(part + u * 32 + lane) & ((1u << lg) - 1u);
+                e[u] = k[u] + ((len * (p + 1)) >> lg);
+                k[u] += (len * p) >> lg;
+            }
         }
-        const int n = n0;
-        if (t.lanes_log2 == 0) {
+        go = more;
+#pragma unroll 1
+        for (bool first = true;; first = false) {
             Vec v[U][D];
-            auto fetch = [&]() {
+            bool rest = false;
 #pragma unroll
-                for (int u = 0; u < U; ++u)
+            for (int u = 0; u < U; ++u)
 #pragma unroll
-                    for (int d = 0; d < D; ++d)
-                        if (c[u].k + d < c[u].e) v[u][d] = __ldg(rec + c[u].k + d);
-            };
-            fetch();
-            if (more) {  // the next batch's offsets, and the ids after it
+                for (int d = 0; d < D; ++d)
+                    if (k[u] + d < e[u]) v[u][d] = __ldg(rec + k[u] + d);
+            if (first && go) {  // behind them, the next parts' offsets and the ids after those
                 offsets();
-                n0 = n1;
-                const bool m2 = src.begin(n1);
-                ids(m2, n1);
-                more = m2;
-            } else {
-                n0 = 0;
-            }
-            for (;;) {
-                bool rest = false;
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-#pragma unroll
-                    for (int d = 0; d < D; ++d)
-                        if (c[u].k + d < c[u].e)
-                            tile_apply_vec<FX, ONE>(a, t, m, v[u][d], c[u].base, c[u].j, lo_rel, span, ev);
-                    c[u].k += D;
-                    rest |= c[u].k < c[u].e;
-                }
-                if (!rest) break;
-                fetch();
-            }
-        } else {
-            const int G = 1 << t.lanes_log2, round = 32 >> t.lanes_log2;
-            const int gl = lane & (G - 1), gq = lane >> t.lanes_log2;
-            if (more) {
-                offsets();
-                n0 = n1;
-                const bool m2 = src.begin(n1);
-                ids(m2, n1);
-                more = m2;
-            } else {
-                n0 = 0;
+                part = done;
+                advance();
+                ids();
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                for (int q0 = 0; q0 < 32 && u * 32 + q0 < n; q0 += round) {
-                    const int q = q0 + gq;
-                    uint32_t k = __shfl_sync(0xffffffffu, c[u].k, q) + gl;
-                    const uint32_t e = __shfl_sync(0xffffffffu, c[u].e, q);
-                    const int base = __shfl_sync(0xffffffffu, c[u].base, q);
-                    const int j = ONE ? 0 : __shfl_sync(0xffffffffu, c[u].j, q);
-                    while (k < e) {
-                        Vec v[D];
 #pragma unroll
-                        for (int d = 0; d < D; ++d)
-                            if (k + d * G < e) v[d] = __ldg(rec + k + d * G);
-#pragma unroll
-                        for (int d = 0; d < D; ++d)
-                            if (k + d * G < e) tile_apply_vec<FX, ONE>(a, t, m, v[d], base, j, lo_rel, span, ev);
-                        k += D * G;
-                    }
-                    __syncwarp();
-                }
+                for (int d = 0; d < D; ++d)
+                    if (k[u] + d < e[u])
+                        tile_apply_vec<FX, ONE>(a, t, m, v[u][d], base[u], j[u], lo_rel, span, ev);
+                k[u] += D;
+                rest |= k[u] < e[u];
             }
+            if (!rest) break;
         }
-        if (!n0) break;
     }
     events += ev;
 }
@@ -639,17 +707,36 @@ __device__ __forceinline__ ulonglong2 ld_head(const ulonglong2* p)
     return v;
 }
 
-// The tile's header of window k (c spikes, the first in `first`) into every
-// tile's mailbox.  Called by the whole block after a block barrier.
-__device__ __forceinline__ void tile_publish(const TileArgs& t, int k, int c, const uint32_t* first, bool fence)
+// The tile's c spikes of window k (the first kTileInline in `first`) into every
+// tile's mailbox, thread r into tile r's.  Called by the whole block after a
+// block barrier.
+__device__ __forceinline__ void tile_publish(const TileArgs& t, int k, int c, const uint32_t* first)
 {
     if ((int)threadIdx.x < t.T) {
-        ulonglong2 h;
-        h.x = ((unsigned long long)(t.epoch + (uint32_t)k) << 32) | (uint32_t)c;
-        h.y = (unsigned long long)first[0] | ((unsigned long long)first[1] << 32);
-        if (fence || c > kTileInline) asm volatile("fence.acq_rel.gpu;" ::: "memory");
-        st_head(t.mail + ((size_t)(k & 1) * t.T + threadIdx.x) * t.T + blockIdx.x, h);
+        ulonglong2* p = t.mail + (((size_t)(k & 1) * t.T + threadIdx.x) * t.T + blockIdx.x) * kTileChunks;
+        const unsigned long long epoch = (unsigned long long)(t.epoch + (uint32_t)k) << 32;
+        if (c > kTileInline) asm volatile("fence.acq_rel.gpu;" ::: "memory");
+        st_head(p, make_ulonglong2(epoch | (uint32_t)c, (unsigned long long)first[0] | ((unsigned long long)first[1] << 32)));
+        if (c > 2 && c <= kTileInline)
+            for (int q = 2; q < c; q += 3)  // (the last chunk may hold stale words past c)
+                st_head(p + 1 + (q - 2) / 3, make_ulonglong2(epoch | first[q], (unsigned long long)first[q + 1] |
+                                                                                 ((unsigned long long)first[q + 2] << 32)));
     }
+}
+
+// A chunk of the wanted epoch, waited for.
+__device__ __forceinline__ ulonglong2 tile_wait(const StepArgs& a, const ulonglong2* p, uint32_t epoch, int* abort_flag)
+{
+    ulonglong2 v = ld_head(p);
+    for (unsigned it = 0; (uint32_t)(v.x >> 32) != epoch; v = ld_head(p)) {
+        if (++it > kBarrierSpins) {
+            atomicOr(a.status, kStatusBarrier);
+            *abort_flag = 1;
+            return make_ulonglong2(0, 0);
+        }
+        if (it > 64) __nanosleep(32);
+    }
+    return v;
 }
 
 // Waits until every tile has published window k.  *n (zero on entry) gets the
@@ -658,39 +745,55 @@ __device__ __forceinline__ void tile_publish(const TileArgs& t, int k, int c, co
 __device__ __forceinline__ bool tile_gather(const StepArgs& a, const TileArgs& t, const TileSmem& m, int k,
                                             const uint32_t* lists, size_t list_len, int* n, int* abort_flag)
 {
-    bool listed = false;  // the tile has more spikes than its header carries
+    bool listed = false;  // the tile has more spikes than its mailbox place holds
     if ((int)threadIdx.x < t.T) {
-        const ulonglong2* p = t.mail + ((size_t)(k & 1) * t.T + blockIdx.x) * t.T + threadIdx.x;
-        ulonglong2 v = ld_head(p);
-        for (unsigned it = 0; (uint32_t)(v.x >> 32) != t.epoch + (uint32_t)k; v = ld_head(p)) {
-            if (++it > kBarrierSpins) {
-                atomicOr(a.status, kStatusBarrier);
-                *abort_flag = 1;
-                v.x = 0;
-                break;
-            }
-            if (it > 64) __nanosleep(32);
-        }
+        const uint32_t epoch = t.epoch + (uint32_t)k;
+        const ulonglong2* p = t.mail + (((size_t)(k & 1) * t.T + blockIdx.x) * t.T + threadIdx.x) * kTileChunks;
+        const ulonglong2 v = tile_wait(a, p, epoch, abort_flag);
         const int c = (int)(uint32_t)v.x;
         int at = 0;
         if (c > 0) {
             at = atomicAdd(n, c);
             listed = c > kTileInline;
             if (listed) asm volatile("fence.acq_rel.gpu;" ::: "memory");
-            if (at + c <= kTileSpikes) {
-                m.spikes[at] = (uint32_t)v.y;
-                if (c > 1) m.spikes[at + 1] = (uint32_t)(v.y >> 32);
+            const bool fits = at + c <= kTileSpikes;
+            uint32_t* out = m.spikes + at;
+            if (fits) {
+                out[0] = (uint32_t)v.y;
+                if (c > 1) out[1] = (uint32_t)(v.y >> 32);
+            }
+            if (!listed) {
+                const int chunks = (c - 2 + 2) / 3;  // after the first
+#pragma unroll 1
+                for (int g = 0; g < chunks; g += 5) {
+                    ulonglong2 w[5];
+#pragma unroll
+                    for (int u = 0; u < 5; ++u)  // in flight together
+                        if (g + u < chunks) w[u] = ld_head(p + 1 + g + u);
+#pragma unroll
+                    for (int u = 0; u < 5; ++u) {
+                        if (g + u >= chunks) continue;
+                        if ((uint32_t)(w[u].x >> 32) != epoch) w[u] = tile_wait(a, p + 1 + g + u, epoch, abort_flag);
+                        const int q = 2 + 3 * (g + u);
+                        if (!fits) continue;
+                        out[q] = (uint32_t)w[u].x;
+                        if (q + 1 < c) out[q + 1] = (uint32_t)w[u].y;
+                        if (q + 2 < c) out[q + 2] = (uint32_t)(w[u].y >> 32);
+                    }
+                }
             }
         }
         m.cnt[threadIdx.x] = c;
         m.at[threadIdx.x] = at;
     }
     const bool any = __syncthreads_or(listed);
-    if (any && *n <= kTileSpikes) {  // eight lanes a tile
+    if (any && *n <= kTileSpikes) {  // the lists, eight lanes a tile
         for (int l = threadIdx.x >> 3; l < t.T; l += blockDim.x >> 3) {
             const int c = m.cnt[l];
+            if (c <= kTileInline) continue;
             const uint32_t* from = lists + (size_t)l * list_len;
-            for (int q = kTileInline + (threadIdx.x & 7); q < c; q += 8) m.spikes[m.at[l] + q] = __ldcg(from + q);
+#pragma unroll 4
+            for (int q = 2 + (threadIdx.x & 7); q < c; q += 8) m.spikes[m.at[l] + q] = __ldcg(from + q);
         }
         __syncthreads();
     }
@@ -704,9 +807,10 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
     __shared__ int abort_flag;
     __shared__ unsigned long long blk_ev;
     __shared__ int count, npg, total;  // the tile's spikes of the window, its POISSON groups, all tiles' spikes
-    __shared__ uint32_t mine[kTileInline];
+    __shared__ uint32_t mine[kTileInline + 2];  // (a chunk's words past the last spike are read)
     __shared__ int scnt[kTileWindow];      // this window's spikes per step
     __shared__ int32_t sbase[2][kTileWindow], stot[kTileWindow + 1];  // places reserved in the steps, the steps' totals
+    __shared__ int32_t ctot[4][kTileWindow];  // the counters' last totals
     const TileSmem m = tile_smem<CUR, FX>(tile_raw, t);
     const int tile = blockIdx.x, tid = threadIdx.x;
     const int64_t s0 = *a.step;
@@ -727,7 +831,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
     {
         uint32_t* z = reinterpret_cast<uint32_t*>(m.ring);
         const int words = (FX ? 4 : 1) * t.R * t.stride;
+#pragma unroll 1
         for (int k = tid; k < words; k += blockDim.x) z[k] = 0;
+#pragma unroll 1
         for (int i = tid; i < t.nl; i += blockDim.x) {
             const int32_t gi = tile_neuron(t, i, tile);
             const bool in = gi < a.ns;
@@ -744,8 +850,10 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
             }
         }
         if (!FX && m.tab)
+#pragma unroll 1
             for (int k = tid; k < 2 * kTileTable; k += blockDim.x) m.tab[k] = t.chain[k];
         if (tid < kTileWindow) scnt[tid] = 0;
+        if (tid < 4 * kTileWindow) ctot[tid / kTileWindow][tid % kTileWindow] = 0;
         if (tid == 0) {
             abort_flag = 0;
             blk_ev = 0;
@@ -764,17 +872,17 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
     {
         const int64_t x0 = s0 - t.R > 0 ? s0 - t.R : 0;
         const int nst = (int)(s0 - x0);
+#pragma unroll 1
         for (int j = tid; j < nst; j += blockDim.x) m.cnt[j] = __ldcg(a.hist_cnt + hs_of(x0 + j));
         __syncthreads();
-        auto get = [&](int l, int q, int& j) {
-            j = l;
-            return __ldcg(a.hist_ids + (size_t)hs_of(x0 + l) * (size_t)a.n_src + q);
-        };
-        tile_deliver<FX, ONE>(a, t, m, x0, (int)(x0 % t.R), lo, hi, TileListed<decltype(get)>(get, m.cnt, nst), ev);
+        TileSource src;
+        src.listed(TileSource::kHistory, nst, hs_of(x0));
+        tile_deliver<FX, ONE>(a, t, m, x0, (int)(x0 % t.R), lo, hi, src, ev);
         if (ONE)  // whole rows, counted by one block a step
             for (int j = tile; j < nst; j += t.T) {
                 const int64_t x = x0 + j;
                 if (x + t.dmin <= lo || x + t.dmin > hi) continue;
+#pragma unroll 1
                 for (int q = tid; q < m.cnt[j]; q += blockDim.x) {
                     const int32_t id = __ldcg(a.hist_ids + (size_t)hs_of(x) * (size_t)a.n_src + q);
                     if (MGC_OK_INDEX(id >= 0 && id < a.n_src))
@@ -787,7 +895,13 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
     // history of the launch's last steps; the counters of the window are final
     const size_t list_len = (size_t)t.nl * t.W;
     auto my_list = [&](int k) { return t.list + ((size_t)(k & 1) * t.T + tile) * list_len; };
+    const int32_t h_end = hs_of(s_end);
+    auto hs_last = [&](int64_t x) {  // history slot of a step less than H before s_end
+        const int32_t h = h_end - (int32_t)(s_end - x);
+        return h < 0 ? h + a.H : h;
+    };
     auto record = [&](int k, int64_t x0, int w, int c) {  // stot, sbase ready; c: this tile's spikes
+#pragma unroll 1
         for (int q = tid; q < c; q += blockDim.x) {
             const uint32_t e = my_list(k)[q];
             const int32_t id = (int32_t)(e & kTileId);
@@ -795,13 +909,13 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
             const int at = atomicAdd(&sbase[k & 1][j], 1);  // any order inside a step
             const int64_t x = x0 + j, rb = rbase + stot[j] + at;
             if (rec && rb < a.raster_ids_cap) a.raster_ids[rb] = id;
-            if (x > s_end - a.H && MGC_OK_INDEX(at < a.n_src)) a.hist_ids[(size_t)hs_of(x) * (size_t)a.n_src + at] = id;
+            if (x > s_end - a.H && MGC_OK_INDEX(at < a.n_src)) a.hist_ids[(size_t)hs_last(x) * (size_t)a.n_src + at] = id;
             if (ONE && x + t.dmin <= hi) ev += (unsigned long long)(a.row_ptr[id + 1] - a.row_ptr[id]);
         }
         if (tile == 0 && tid < w) {
             const int64_t x = x0 + tid;
             const int c_all = stot[tid + 1] - stot[tid];
-            if (x > s_end - a.H) a.hist_cnt[hs_of(x)] = c_all;
+            if (x > s_end - a.H) a.hist_cnt[hs_last(x)] = c_all;
             if (rec) {
                 if (x - rstep0 < a.raster_steps_cap)
                     a.raster_counts[x - rstep0] = c_all;
@@ -815,7 +929,12 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
     // running sums of window k's step totals, by the first warp
     auto totals = [&](int k, int w) {
         if (tid < 32) {
-            int c = tid < w ? __ldcg(t.cnt + (k & 3) * kTileWindow + tid) : 0;
+            int c = 0;
+            if (tid < w) {
+                const int32_t now = __ldcg(tile_counter(t, k, tid));
+                c = now - ctot[k & 3][tid];
+                ctot[k & 3][tid] = now;
+            }
 #pragma unroll
             for (int o = 1; o < kTileWindow; o <<= 1) {
                 const int v = __shfl_up_sync(0xffffffffu, c, o);
@@ -832,32 +951,27 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
         const int wl = (int)(s_end - w0 < t.W ? s_end - w0 : t.W);
         if (n_pg) tile_poisson(a, t, m, w0, wl, n_pg, my_list(k), mine, &count, scnt);
         tile_update<CUR, FX>(a, t, m, w0, wl, slot, t.ahead && k == 0, my_list(k), mine, &count, scnt);
-        if (tile == 0 && tid < kTileWindow) t.cnt[((k + 1) & 3) * kTileWindow + tid] = 0;
         __syncthreads();
         const int c_now = count;
-        tile_publish(t, k, c_now, mine, tile == 0);  // (tile 0 cleared counters)
+        tile_publish(t, k, c_now, mine);
         // the steps' places for this tile's spikes, needed a window later
         int place = 0;
         if (tid >= 32 && tid < 32 + wl && scnt[tid - 32])
-            place = atomicAdd(t.cnt + (k & 3) * kTileWindow + tid - 32, scnt[tid - 32]);
+            place = atomicAdd(tile_counter(t, k, tid - 32), scnt[tid - 32]);
         const uint32_t* lists = t.list + (size_t)(k & 1) * t.T * list_len;
         if (!tile_gather(a, t, m, k, lists, list_len, &total, &abort_flag)) return;
         if (tid >= 32 && tid < 32 + kTileWindow) {
-            sbase[k & 1][tid - 32] = place;
+            sbase[k & 1][tid - 32] = place - ctot[k & 3][tid - 32];
             scnt[tid - 32] = 0;
         }
         if (tid == 0) count = 0;
         if (k > 0) totals(k - 1, w_prev);
-        if (total <= kTileSpikes) {
-            tile_deliver<FX, ONE>(a, t, m, w0, slot, lo, hi, TileGathered(m.spikes, total), ev);
-        } else {
-            auto get = [&](int l, int q, int& j) {
-                const uint32_t e = __ldcg(lists + (size_t)l * list_len + q);
-                j = (int)(e >> kTileStepShift);
-                return (int32_t)(e & kTileId);
-            };
-            tile_deliver<FX, ONE>(a, t, m, w0, slot, lo, hi, TileListed<decltype(get)>(get, m.cnt, t.T), ev);
-        }
+        TileSource src;
+        if (total <= kTileSpikes)
+            src.gathered(total);
+        else
+            src.listed(TileSource::kTiles, t.T, k);
+        tile_deliver<FX, ONE>(a, t, m, w0, slot, lo, hi, src, ev);
         __syncthreads();
         if (tid == 0) total = 0;
         if (k > 0) record(k - 1, w0 - w_prev, w_prev, c_prev);
@@ -868,12 +982,13 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
         if (slot >= t.R) slot -= t.R;
     }
     // the last window's raster and history: an empty window makes its counters final
-    tile_publish(t, k, 0, mine, true);
+    tile_publish(t, k, 0, mine);
     if (!tile_gather(a, t, m, k, t.list, 0, &total, &abort_flag)) return;
     totals(k - 1, w_prev);
     __syncthreads();
     record(k - 1, w0 - w_prev, w_prev, c_prev);
     // back to the single-step form: the state, and the arrivals of s_end
+#pragma unroll 1
     for (int i = tid; i < t.nl; i += blockDim.x) {
         const int32_t gi = tile_neuron(t, i, tile);
         if (gi >= a.ns) continue;
@@ -905,11 +1020,11 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
     if (last_block(a.done) && tid == 0) {
         if (rec) *a.raster_pos = rbase;
         if (a.ev_mark) *a.ev_mark = *(volatile unsigned long long*)a.events;
-        a.hist_cnt[hs_of(s_end)] = 0;
-        for (int j = 0; j < 4 * kTileWindow; ++j) t.cnt[j] = 0;
+        a.hist_cnt[h_end] = 0;
+        for (int j = 0; j < 4 * kTileWindow; ++j) t.cnt[j * kTileLine] = 0;
         *a.done = 0;
         a.slots[0] = (int32_t)((slot0 + nsteps) % a.M);
-        a.slots[1] = hs_of(s_end);
+        a.slots[1] = h_end;
         *a.step = s_end;
     }
 }
@@ -930,7 +1045,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
 //
 // Bound by the step's chain of dependent accesses: exchange, segment
 // offsets, records, and after a spike of its own the incoming list and its
-// weights.  784 -> 1,600 plastic network, 1.9e4 events a step: see DESIGN.
+// weights.  784 -> 1,600 plastic network, 1.9e4 events a step: 12.1 us a step
+// with the single-step ring kernels, 5.2 here.
 // ---------------------------------------------------------------------------
 struct TileStdpSmem {
     int32_t* lf;       // [n] last spike of every neuron
@@ -951,9 +1067,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_stdp(StepArgs a, TileA
     __shared__ int abort_flag;
     __shared__ unsigned long long blk_ev;
     __shared__ int count, npg, total;
-    __shared__ uint32_t mine[kTileInline];
+    __shared__ uint32_t mine[kTileInline + 2];
     __shared__ int scnt[kTileWindow];
-    __shared__ int32_t sbase[2], stot;   // places reserved in a step, a step's spikes
+    __shared__ int32_t sbase[2], stot, ctot[4];   // places reserved in a step, a step's spikes, the counters' totals
     const TileSmem m = tile_smem<CUR, true>(tile_raw, t);
     TileStdpSmem q;
     {
@@ -977,6 +1093,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_stdp(StepArgs a, TileA
                                     reinterpret_cast<unsigned long long*>(a.ring_i)};
 
     // state of the tile, the pending input of steps s0 .. s0 + R - 1
+#pragma unroll 1
     for (int i = tid; i < t.nl; i += blockDim.x) {
         const int32_t gi = tile_neuron(t, i, tile);
         const bool in = gi < a.ns;
@@ -997,6 +1114,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_stdp(StepArgs a, TileA
     for (int i = tid; i < (a.n + 31) / 32; i += blockDim.x) q.fired[i] = 0;
     for (int i = tid; i <= t.nl; i += blockDim.x) q.in_off[i] = t.in_off[(size_t)tile * t.nl + i];
     if (tid < kTileWindow) scnt[tid] = 0;
+    if (tid < 4) ctot[tid] = 0;
     if (tid == 0) {
         abort_flag = 0;
         blk_ev = 0;
@@ -1016,15 +1134,24 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_stdp(StepArgs a, TileA
     // `width` of them) in turn
     auto each_spike = [&](int k, int group, int groups, auto f) {
         if (total <= kTileSpikes) {
+#pragma unroll 1
             for (int x = group; x < total; x += groups) f((int32_t)(m.spikes[x] & kTileId));
         } else {
-            const uint32_t* lists = t.list + (size_t)(k & 1) * t.T * list_len;
+#pragma unroll 1
             for (int l = 0; l < t.T; ++l)
-                for (int x = group; x < m.cnt[l]; x += groups) f((int32_t)(__ldcg(lists + (size_t)l * list_len + x) & kTileId));
+#pragma unroll 1
+                for (int x = group; x < m.cnt[l]; x += groups)
+                    f((int32_t)((m.cnt[l] > kTileInline ? __ldcg(tile_list(t, k, l) + x) : tile_mail(t, k, l, x)) & kTileId));
         }
+    };
+    auto total_of = [&](int k) {  // step k's spikes (one thread, its counter final)
+        const int32_t now = __ldcg(tile_counter(t, k, 0));
+        stot = now - ctot[k & 3];
+        ctot[k & 3] = now;
     };
     // raster places of step x's spikes (the step's counter is final), one step late
     auto record = [&](int k, int64_t x, int c) {
+#pragma unroll 1
         for (int y = tid; y < c; y += blockDim.x) {
             const int32_t id = (int32_t)(my_list(k)[y] & kTileId);
             const int64_t rb = rbase + atomicAdd(&sbase[k & 1], 1);  // any order inside a step
@@ -1045,20 +1172,19 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_stdp(StepArgs a, TileA
     for (int64_t s = s0; s < s_end; ++s, ++k) {
         if (n_pg) tile_poisson(a, t, m, s, 1, n_pg, my_list(k), mine, &count, scnt);
         tile_update<CUR, true>(a, t, m, s, 1, slot, false, my_list(k), mine, &count, scnt);
-        if (tile == 0 && tid == 0) t.cnt[((k + 1) & 3) * kTileWindow] = 0;
         __syncthreads();
         const int c_now = count;
-        tile_publish(t, k, c_now, mine, tile == 0);  // (tile 0 cleared a counter)
+        tile_publish(t, k, c_now, mine);
         int place = 0;
-        if (tid == 32 && c_now) place = atomicAdd(t.cnt + (k & 3) * kTileWindow, c_now);
+        if (tid == 32 && c_now) place = atomicAdd(tile_counter(t, k, 0), c_now);
         if (!tile_gather(a, t, m, k, t.list + (size_t)(k & 1) * t.T * list_len, list_len, &total, &abort_flag)) return;
         if (tid == 32) {
-            sbase[k & 1] = place;
+            sbase[k & 1] = place - ctot[k & 3];
             scnt[0] = 0;
         }
         if (tid == 0) {
             count = 0;
-            if (k > 0) stot = __ldcg(t.cnt + ((k - 1) & 3) * kTileWindow);
+            if (k > 0) total_of(k - 1);
         }
         each_spike(k, tid, blockDim.x, [&](int32_t id) {
             if (!MGC_OK_INDEX(id >= 0 && id < a.n)) return;
@@ -1072,6 +1198,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_stdp(StepArgs a, TileA
             const uint32_t* o = t.off + (size_t)id * t.T + tile;
             const uint32_t b = __ldg(o), e = __ldg(o + 1);
             if (!MGC_OK_INDEX(b <= e && e <= t.n_vec)) return;
+#pragma unroll 1
             for (uint32_t r0 = b + (lane & 7); r0 < e; r0 += 32) {
                 uint2 x[4];
                 uint32_t cp[4];
@@ -1101,9 +1228,10 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_stdp(StepArgs a, TileA
         });
         // the plastic synapses onto this tile's spiking neurons, the block on each
         for (int y = 0; y < c_now; ++y) {
-            const int32_t id = (int32_t)((y < kTileInline ? mine[y] : __ldcg(my_list(k) + y)) & kTileId);
+            const int32_t id = (int32_t)((y < kTileInline ? mine[y] : __ldcg(my_list(k) + y)) & kTileId);  // (uniform)
             const int g = id >> 2, local = g / t.T * 4 + (id & 3);
             const uint32_t e = q.in_off[local + 1];
+#pragma unroll 1
             for (uint32_t p0 = q.in_off[local] + tid; p0 < e; p0 += 2 * blockDim.x) {
                 uint2 en[2];
                 uint32_t w[2], cp[2];
@@ -1141,11 +1269,12 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_stdp(StepArgs a, TileA
     }
     // the last step's raster: an empty window makes its counter final
     __syncthreads();
-    tile_publish(t, k, 0, mine, true);
+    tile_publish(t, k, 0, mine);
     if (!tile_gather(a, t, m, k, t.list, 0, &total, &abort_flag)) return;
-    if (tid == 0) stot = __ldcg(t.cnt + ((k - 1) & 3) * kTileWindow);
+    if (tid == 0) total_of(k - 1);
     __syncthreads();
     record(k - 1, s_end - 1, c_prev);
+#pragma unroll 1
     for (int i = tid; i < t.nl; i += blockDim.x) {
         const int32_t gi = tile_neuron(t, i, tile);
         if (gi >= a.ns) continue;
@@ -1170,7 +1299,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_stdp(StepArgs a, TileA
     if (tid == 0 && blk_ev) atomicAdd(a.events, blk_ev);
     if (last_block(a.done) && tid == 0) {
         if (rec_on) *a.raster_pos = rbase;
-        for (int j = 0; j < 4 * kTileWindow; ++j) t.cnt[j] = 0;
+        for (int j = 0; j < 4 * kTileWindow; ++j) t.cnt[j * kTileLine] = 0;
         *a.done = 0;
         a.slots[0] = (int32_t)((slot0 + nsteps) % a.M);
         *a.step = s_end;

@@ -180,3 +180,14 @@ def test_tiles_in_fixed_point_on_request():
         outs.append((sim.read_raster(), sim.state(), sim.info()))
         sim.close()
     same(*outs)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx,delays", [(2, [1]), (3, [1]), (5, [3, 4]), (148 * 44 + 3, [1]), (148 * 44 + 4, [1]),
+                                       (148 * 12, [4, 6]), (148 * 12 - 4, [4, 6])])
+def test_tiles_mailbox_edges(nx, delays):
+    """Inputs that fire in every step fill a tile's mailbox place to a chunk's edge
+    (2 and 3 spikes, 5 and 6), to its last spike and one beyond (47 and 48)."""
+    spec = dict(n=61, nx=nx, k=40, delays=delays, rate=1.0)
+    ref = run(spec, [100, 57], [0, None], {})
+    same(ref, run(spec, [100, 57], [None, None], {}))
