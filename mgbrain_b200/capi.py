@@ -228,6 +228,17 @@ def check(status):
         raise MgcError(status, lib().mgc_last_error().decode())
 
 
+def _cut(a, n):
+    """The first n entries of a new array; the (mostly untouched) capacity is not
+    kept.  Long results are cut in place (6.3e6 ids: their copy took 3.2 ms, a
+    pass of a 1.1e6-neuron network 75.9 ms with it and 71.5 without); a short
+    one is copied, which costs less than giving back part of a mapping."""
+    if n * a.itemsize < 1 << 18:
+        return a[:n].copy()
+    a.resize(n, refcheck=False)
+    return a
+
+
 def _ptr(a):
     return None if a is None else a.ctypes.data_as(C.c_void_p)
 
@@ -472,8 +483,7 @@ class Simulator:
         first, ns, ni = C.c_int64(), C.c_int64(), C.c_int64()
         check(lib().mgc_read_raster(self._h, C.byref(first), _ptr(counts), max_steps, _ptr(ids),
                                     max_ids, C.byref(ns), C.byref(ni)))
-        # copies: the (mostly untouched) capacity buffers are not kept alive
-        return first.value, counts[:ns.value].copy(), ids[:ni.value].copy()
+        return first.value, _cut(counts, ns.value), _cut(ids, ni.value)
 
     def stage_raster(self):
         """Enqueues a device copy of the raster so far and starts a new one
@@ -489,7 +499,7 @@ class Simulator:
         first, ns, ni = C.c_int64(), C.c_int64(), C.c_int64()
         check(lib().mgc_raster_collect(self._h, C.byref(first), _ptr(counts), max_steps, _ptr(ids),
                                        max_ids, C.byref(ns), C.byref(ni)))
-        return first.value, counts[:ns.value].copy(), ids[:ni.value].copy()
+        return first.value, _cut(counts, ns.value), _cut(ids, ni.value)
 
     def state(self):
         n = self.n
