@@ -254,7 +254,7 @@ mgc_status build_tiles(mgc_sim* s)
     // at most one vector in each segment is not full
     const size_t most = ((size_t)s->S / 2 + (size_t)s->n * T) * vec_bytes;
     const int W = stdp ? 1 : std::min(kTileWindow, s->dmin);
-    const size_t need = most + (stdp ? 12 * (size_t)s->S : 0) + ((size_t)s->n * T + 1) * 4 + 2 * (size_t)W * nl_of(T) * T * 4 + 32 * (size_t)T * T * kTileChunks + 16 * (size_t)a.ns;
+    const size_t need = most + (stdp ? 12 * (size_t)s->S : 0) + ((size_t)s->n * T + 1) * 4 + kTileLists * (size_t)W * nl_of(T) * T * 4 + 32 * (size_t)T * T * kTileChunks + 16 * (size_t)a.ns;
     // offsets in vectors, and in records while they are filled
     if ((int64_t)s->n * T + 1 > (int64_t)0x7fffffff || most / vec_bytes > kIndex / 2) return MGC_OK;
     size_t free_b = 0, total_b = 0;
@@ -273,7 +273,7 @@ mgc_status build_tiles(mgc_sim* s)
     float *we = nullptr, *wi = nullptr, *chain = nullptr;
     CKS(s->alloc(&off, (size_t)s->n * T + 1, false));
     t.off = off;
-    CKS(s->alloc(&t.list, 2 * (size_t)T * t.nl * W, false));
+    CKS(s->alloc(&t.list, kTileLists * (size_t)T * t.nl * W, false));
     CKS(s->alloc(&t.mail, 2 * (size_t)T * T * kTileChunks));
     t.epoch = 1;
     CKS(s->alloc(&t.cnt, 4 * kTileWindow * kTileLine));

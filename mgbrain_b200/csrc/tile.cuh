@@ -48,14 +48,18 @@
 // chunk carries the epoch, so none has to be ordered after another, and no
 // fence is needed; thread l of a block polls the place of tile l in its own
 // mailbox, which no other block reads, so no counter or line is shared.  Only a
-// tile with more spikes than a mailbox holds sends just the count and writes
-// them to its list of buffer k & 1, with a fence before and at its readers.
+// tile with more spikes than a mailbox holds sends just the count; they are in
+// its list of buffer k % kTileLists, with a fence before and at its readers.
 // (11,000 neurons: 5.0 us an exchange with one set of headers polled by all
 // blocks and release stores, 2.1 with mailboxes; 44,700 neurons, 13 spikes a
 // tile and window: 8.0 us with two spikes a header and fenced lists.)  A tile
-// overwrites a buffer two windows later, when every tile has published the
-// window between, which it does after reading the buffer.  Waits are bounded
-// (kStatusBarrier).
+// overwrites a mailbox place two windows later, when every tile has published
+// the window between, which it does after reading the place.  A list is read a
+// second time, by its own tile's raster writes at the end of the window after
+// its own; no block barrier lies between those and the next window's updates,
+// which write the list of two windows on.  So there are three list buffers, not
+// two: the buffer of window k is written again in window k + 3, behind the
+// barriers of window k + 2.  Waits are bounded (kStatusBarrier).
 //
 // Raster: a step's place in it needs the step's spikes of all tiles, so each
 // tile adds its counts to the window's 16 step counters when it publishes,
@@ -96,7 +100,7 @@ struct TileArgs {
     const float* we;      // [ns] weight per sign of each neuron (fp32 sums)
     const float* wi;
     const float* chain;   // [2][kTileTable] sums of k weights (exc, inh), when table
-    uint32_t* list;       // [2][T][nl*W] spikes of a window: id | step in the window << 28
+    uint32_t* list;       // [kTileLists][T][nl*W] spikes of a window: id | step in the window << 28
     ulonglong2* mail;     // [2][T reader][T][kTileChunks]
     uint32_t epoch;       // epoch of the launch's first window (they count on over the launches)
     int32_t* cnt;         // [4][kTileWindow] counters (tile_counter) of a window's steps' spikes; zero between launches
@@ -110,6 +114,7 @@ constexpr int kTileLine = 32;       // a counter has a line to itself: 148 block
                                     // on one line those atomics queued for 8 to 70 us a window
 constexpr int kTileChunks = 16;     // chunks of a mailbox place
 constexpr int kTileInline = 2 + 3 * (kTileChunks - 1);  // spikes they carry
+constexpr int kTileLists = 3;       // list buffers (see the exchange above)
 constexpr int kTileSpikes = 8192;   // spikes of a window gathered in shared memory; every mailbox full fits
 constexpr int kMaxTiles = kTileSpikes / kTileInline;
 constexpr int kTileStepShift = 28;  // spike word: id below, step in the window above
@@ -480,10 +485,10 @@ constexpr int kTileD = 4;           // 8-byte vectors of each it loads at once (
 constexpr int kTileBatch = 32 * kTileU;
 constexpr uint32_t kTileId = (1u << kTileStepShift) - 1u;
 
-// Tile l's list in window k, and spike q of the tile from its mailbox place.
+// Tile l's list of window k, and spike q of the tile from its mailbox place.
 __device__ __forceinline__ const uint32_t* tile_list(const TileArgs& t, int k, int l)
 {
-    return t.list + ((size_t)(k & 1) * t.T + l) * ((size_t)t.nl * t.W);
+    return t.list + ((size_t)(k % kTileLists) * t.T + l) * ((size_t)t.nl * t.W);
 }
 __device__ __forceinline__ uint32_t tile_mail(const TileArgs& t, int k, int l, int q)
 {
@@ -894,7 +899,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
     // the spikes of window k (w steps from x0): their raster places, and the
     // history of the launch's last steps; the counters of the window are final
     const size_t list_len = (size_t)t.nl * t.W;
-    auto my_list = [&](int k) { return t.list + ((size_t)(k & 1) * t.T + tile) * list_len; };
+    auto my_list = [&](int k) { return t.list + ((size_t)(k % kTileLists) * t.T + tile) * list_len; };
     const int32_t h_end = hs_of(s_end);
     auto hs_last = [&](int64_t x) {  // history slot of a step less than H before s_end
         const int32_t h = h_end - (int32_t)(s_end - x);
@@ -958,7 +963,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
         int place = 0;
         if (tid >= 32 && tid < 32 + wl && scnt[tid - 32])
             place = atomicAdd(tile_counter(t, k, tid - 32), scnt[tid - 32]);
-        const uint32_t* lists = t.list + (size_t)(k & 1) * t.T * list_len;
+        const uint32_t* lists = t.list + (size_t)(k % kTileLists) * t.T * list_len;
         if (!tile_gather(a, t, m, k, lists, list_len, &total, &abort_flag)) return;
         if (tid >= 32 && tid < 32 + kTileWindow) {
             sbase[k & 1][tid - 32] = place - ctot[k & 3][tid - 32];
@@ -1129,7 +1134,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_stdp(StepArgs a, TileA
     __syncthreads();
     const int n_pg = npg;
     const size_t list_len = (size_t)t.nl * t.W;
-    auto my_list = [&](int k) { return t.list + ((size_t)(k & 1) * t.T + tile) * list_len; };
+    auto my_list = [&](int k) { return t.list + ((size_t)(k % kTileLists) * t.T + tile) * list_len; };
     // f(id) for every spike of the step, the block's threads (or groups of
     // `width` of them) in turn
     auto each_spike = [&](int k, int group, int groups, auto f) {
@@ -1177,7 +1182,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_stdp(StepArgs a, TileA
         tile_publish(t, k, c_now, mine);
         int place = 0;
         if (tid == 32 && c_now) place = atomicAdd(tile_counter(t, k, 0), c_now);
-        if (!tile_gather(a, t, m, k, t.list + (size_t)(k & 1) * t.T * list_len, list_len, &total, &abort_flag)) return;
+        if (!tile_gather(a, t, m, k, tile_list(t, k, 0), list_len, &total, &abort_flag)) return;
         if (tid == 32) {
             sbase[k & 1] = place - ctot[k & 3];
             scnt[0] = 0;

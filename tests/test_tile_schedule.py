@@ -1,0 +1,233 @@
+"""The tiled step group's windows (k_tile), restated on the CPU: blocks of warps
+in random interleavings, with the kernel's list buffers, mailboxes, step counters
+and block barriers, and nothing else between them.  Every block must deliver each
+window's spikes exactly once, and every spike must get a raster place of its own
+in its own window.
+
+The number of list buffers is the kernel's (kTileLists).  With two, a warp that
+has no spike left to record starts the next window's update and overwrites
+entries that a slower warp of the block has yet to read; the restatement shows
+that."""
+import os
+import random
+import re
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+SOURCE = open(os.path.join(ROOT, "mgbrain_b200", "csrc", "tile.cuh")).read()
+
+WARPS = 3      # warp 0 publishes, polls and sums the counters; warp 1 reserves the places
+INLINE = 2     # spikes a mailbox place holds
+GATHERED = 12  # spikes of a window that fit in shared memory
+SLOTS = 4      # counters
+
+
+class Failure(Exception):
+    pass
+
+
+class Block:
+    def __init__(self, tiles):
+        self.count = self.total = 0
+        self.mine = [None] * INLINE
+        self.cnt = [0] * tiles
+        self.spikes = []
+        self.ctot = [0] * SLOTS
+        self.sbase = [0, 0]
+        self.stot = 0
+        self.arrived = 0
+        self.generation = 0
+        self.delivered = []     # per window
+
+
+class Group:
+    """One launch of `windows` windows over `tiles` blocks; load[k][b][w]: spikes
+    of warp w of block b in window k."""
+
+    def __init__(self, load, lists, seed):
+        self.load, self.lists = load, lists
+        self.windows, self.tiles = len(load), len(load[0])
+        self.rng = random.Random(seed)
+        self.list = [[[] for _ in range(self.tiles)] for _ in range(lists)]
+        self.mail = [[[(-1, 0, ())] * self.tiles for _ in range(self.tiles)] for _ in range(2)]  # [parity][reader][tile]
+        self.counter = [0] * SLOTS
+        self.raster = [{} for _ in range(self.windows)]
+        self.blocks = [Block(self.tiles) for _ in range(self.tiles)]
+
+    def spike(self, k, b, w, i):
+        return (k, b, w, i)
+
+    def barrier(self, blk):
+        blk.arrived += 1
+        g = blk.generation
+        if blk.arrived == WARPS:
+            blk.arrived = 0
+            blk.generation += 1
+        while blk.generation == g:
+            yield False            # waits: no progress
+
+    def put(self, b, k, pos, e):
+        row = self.list[k % self.lists][b]
+        row.extend([None] * (pos + 1 - len(row)))
+        row[pos] = e
+
+    def record(self, k, b, w, c):
+        blk = self.blocks[b]
+        for q in range(w, c, WARPS):
+            e = self.list[k % self.lists][b][q]
+            yield True
+            at = blk.sbase[k & 1]
+            blk.sbase[k & 1] += 1
+            if e is None or e[0] != k or e[1] != b:
+                raise Failure(f"window {k}, tile {b}: entry {q} of its list is {e}")
+            if at in self.raster[k] or not 0 <= at < blk.stot:
+                raise Failure(f"window {k}: place {at} of {blk.stot}")
+            self.raster[k][at] = e
+            yield True
+
+    def totals(self, k, blk):
+        now = self.counter[k % SLOTS]
+        blk.stot = now - blk.ctot[k % SLOTS]
+        blk.ctot[k % SLOTS] = now
+
+    def gather(self, k, b, w):
+        """tile_gather: polled by warp 0; long lists copied by all warps."""
+        blk = self.blocks[b]
+        if w == 0:
+            blk.spikes = [None] * GATHERED
+            for l in range(self.tiles):
+                while self.mail[k & 1][b][l][0] != k:
+                    yield False
+                _, c, first = self.mail[k & 1][b][l]
+                at = blk.total
+                blk.total += c
+                blk.cnt[l] = (c, at)
+                if at + c <= GATHERED and c <= INLINE:
+                    blk.spikes[at:at + c] = first[:c]
+                yield True
+        yield from self.barrier(blk)
+        if blk.total <= GATHERED and any(c > INLINE for c, _ in blk.cnt):
+            for l in range(w, self.tiles, WARPS):
+                c, at = blk.cnt[l]
+                if c > INLINE:
+                    for q in range(c):
+                        blk.spikes[at + q] = self.list[k % self.lists][l][q]
+                        yield True
+            yield from self.barrier(blk)
+
+    def publish(self, k, b, c):
+        blk = self.blocks[b]
+        for r in range(self.tiles):
+            self.mail[k & 1][r][b] = (k, c, tuple(blk.mine))
+            yield True
+
+    def warp(self, b, w):
+        blk = self.blocks[b]
+        c_prev = 0
+        for k in range(self.windows):
+            for i in range(self.load[k][b][w]):         # the update's spikes
+                pos = blk.count
+                blk.count += 1
+                yield True
+                e = self.spike(k, b, w, i)
+                if pos < INLINE:
+                    blk.mine[pos] = e
+                self.put(b, k, pos, e)
+                yield True
+            yield from self.barrier(blk)
+            c_now = blk.count
+            yield True
+            place = 0
+            if w == 0:
+                yield from self.publish(k, b, c_now)
+            if w == 1:
+                place = self.counter[k % SLOTS]
+                self.counter[k % SLOTS] += c_now
+                yield True
+            yield from self.gather(k, b, w)
+            if w == 1:
+                blk.sbase[k & 1] = place - blk.ctot[k % SLOTS]
+            if w == 0:
+                blk.count = 0
+                if k > 0:
+                    self.totals(k - 1, blk)
+            yield True
+            if blk.total <= GATHERED:                    # the delivery
+                for q in range(w, blk.total, WARPS):
+                    blk.delivered.append(blk.spikes[q])
+                    yield True
+            else:
+                for l in range(self.tiles):
+                    c, _ = blk.cnt[l]
+                    for q in range(w, c, WARPS):
+                        blk.delivered.append(self.list[k % self.lists][l][q] if c > INLINE
+                                             else self.mail[k & 1][b][l][2][q])
+                        yield True
+            yield from self.barrier(blk)
+            if w == 0:
+                blk.total = 0
+            if k > 0:
+                yield from self.record(k - 1, b, w, c_prev)
+            c_prev = c_now
+        k = self.windows
+        if w == 0:
+            yield from self.publish(k, b, 0)
+        yield from self.gather(k, b, w)
+        if w == 0:
+            self.totals(k - 1, blk)
+        yield from self.barrier(blk)
+        yield from self.record(k - 1, b, w, c_prev)
+
+    def run(self):
+        live = [self.warp(b, w) for b in range(self.tiles) for w in range(WARPS)]
+        weight = [1] * len(live)
+        idle = 0
+        while live:
+            if self.rng.random() < 0.05:                 # some warps run ahead of the others for a while
+                weight = [self.rng.choice((1, 1, 30)) for _ in live]
+            i = self.rng.choices(range(len(live)), weight[:len(live)])[0]
+            try:
+                idle = 0 if next(live[i]) else idle + 1
+            except StopIteration:
+                live.pop(i)
+            if idle > 100_000:
+                raise Failure("every warp waits")
+        for k in range(self.windows):
+            want = {self.spike(k, b, w, i) for b in range(self.tiles) for w in range(WARPS)
+                    for i in range(self.load[k][b][w])}
+            if set(self.raster[k].values()) != want or len(self.raster[k]) != len(want):
+                raise Failure(f"window {k}: raster {sorted(self.raster[k].values())}")
+        want = sorted(self.spike(k, b, w, i) for k in range(self.windows) for b in range(self.tiles)
+                      for w in range(WARPS) for i in range(self.load[k][b][w]))
+        for b, blk in enumerate(self.blocks):
+            if sorted(blk.delivered) != want:
+                raise Failure(f"tile {b} delivered other spikes")
+
+
+def loads(seed):
+    rng = random.Random(seed)
+    tiles = rng.choice((1, 2, 3))
+    most = rng.choice((1, 3, 6))
+    return [[[rng.randint(0, most) for _ in range(WARPS)] for _ in range(tiles)] for _ in range(rng.randint(1, 6))]
+
+
+def kernel_lists():
+    m = re.search(r"constexpr int kTileLists = (\d+);", SOURCE)
+    return int(m.group(1)) if m else 2      # (buffer k & 1 before there was a constant)
+
+
+@pytest.mark.parametrize("chunk", range(8))
+def test_windows_deliver_and_record_every_spike_once(chunk):
+    for seed in range(60 * chunk, 60 * (chunk + 1)):
+        Group(loads(seed), kernel_lists(), seed).run()
+
+
+def test_two_list_buffers_would_not_do():
+    failed = 0
+    for seed in range(200):
+        try:
+            Group(loads(seed), 2, seed).run()
+        except Failure:
+            failed += 1
+    assert failed > 0
