@@ -736,8 +736,7 @@ mgc_status launch_shapes(mgc_sim* s)
             for (int wide = 0; wide < 2; ++wide)
                 for (int v = 0; v < 2; ++v) {
                     for (int pl = 0; pl < 2; ++pl)
-                        CK(cudaFuncSetAttribute((const void*)window_kernel(s, v, wide, pl),
-                                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s->window_smem[wide]));
+                        CKS(allow_shared((const void*)window_kernel(s, v, wide, pl), s->device));
                     // both forms of a variant are compiled for the same blocks per SM
                     const WindowKernel k = window_kernel(s, v, wide, false);
                     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, kPushBlock, s->window_smem[wide]));

@@ -64,6 +64,16 @@ mgc_status device_attr(cudaDeviceAttr attr, int device, int* value)
     return MGC_OK;
 }
 
+mgc_status allow_shared(const void* kernel, int device)
+{
+    int optin = 0;
+    CKS(device_attr(cudaDevAttrMaxSharedMemoryPerBlockOptin, device, &optin));
+    cudaFuncAttributes f;
+    CK(cudaFuncGetAttributes(&f, kernel));
+    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)f.sharedSizeBytes));
+    return MGC_OK;
+}
+
 
 const char* last_error_text() { return g_last_error.c_str(); }
 

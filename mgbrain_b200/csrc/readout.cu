@@ -495,7 +495,7 @@ mgc_status mgc_partition_stats(mgc_sim* s, const int32_t* part, int32_t nparts, 
     cudaDeviceProp prop;
     CK(cudaGetDeviceProperties(&prop, s->device));
     const size_t smem = 4 * 3 * (size_t)nparts;
-    if (smem > 48 * 1024) CK(cudaFuncSetAttribute(k_partition_stats, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) CKS(allow_shared((const void*)k_partition_stats, s->device));
     // a partition handle's targets are local ids; their zones are those of
     // the whole-network ids from its first neuron on
     k_partition_stats<<<prop.multiProcessorCount * 4, 256, smem, s->stream>>>(s->a.row_ptr, s->a.syn, n, s->a.tmask,

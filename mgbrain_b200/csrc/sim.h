@@ -204,6 +204,11 @@ namespace mgc {
 // One attribute of the device (cudaGetDeviceProperties reads them all: 5 ms a call).
 mgc_status device_attr(cudaDeviceAttr attr, int device, int* value);
 
+// Lets launches of `kernel` use all the shared memory a block may have.  The
+// limit belongs to the kernel in the context, not to a handle: one set to a
+// handle's own need would refuse the launches of a larger handle built before.
+mgc_status allow_shared(const void* kernel, int device);
+
 // Temporary device buffer freed on scope exit.
 struct DevTmp {
     void* p = nullptr;

@@ -352,8 +352,7 @@ mgc_status build_tiles(mgc_sim* s)
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(s->stream));
         s->tile_smem = tile_stdp_bytes(t.nl, t.R, T, cur, s->n);
-        CK(cudaFuncSetAttribute((const void*)tile_kernel(s), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)s->tile_smem));
+        CKS(allow_shared((const void*)tile_kernel(s), s->device));
         s->tile_ok = s->tile_on = true;
         s->tile_stale = false;
         return MGC_OK;
@@ -366,8 +365,7 @@ mgc_status build_tiles(mgc_sim* s)
     CK(cudaGetLastError());
     s->tile_one = one;
     s->tile_smem = tile_smem_bytes(t.nl, t.R, T, fx, cur, t.table != 0);
-    CK(cudaFuncSetAttribute((const void*)tile_kernel(s), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)s->tile_smem));
+    CKS(allow_shared((const void*)tile_kernel(s), s->device));
     s->tile_ok = s->tile_on = true;
     return MGC_OK;
 }
