@@ -324,6 +324,14 @@ mgc_status mgc_fault_inject_alloc(int64_t n);
  * reference counterpart (the reference has no waits inside kernels). */
 mgc_status mgc_selftest_wait_timeout(int32_t device, int32_t which, int32_t* status, double* ms);
 
+/* Self-test of the tiled step group's waits, with no fault: launches it on the
+ * handle without the last tile's block, so that the other blocks' waits run out
+ * (about a second; every access stays in its arrays).  mgc_sync then returns
+ * MGC_ERR_CUDA, and later launches of the group do nothing, until a checkpoint is
+ * loaded.  MGC_ERR_INVALID for a handle whose steps do not run in that group on
+ * two or more tiles.  No reference counterpart. */
+mgc_status mgc_selftest_tile_timeout(mgc_sim* sim);
+
 /* Enqueues `steps` steps on the handle's stream and returns without
  * waiting.  Replaces the step loop of MGSimulator::simulate_sparse
  * (mgsim.cpp:794-857) calling mgsim_step_sparse (mgcore.cu:535-554);

@@ -37,7 +37,7 @@ EXPORTED = (
     "mgc_create_partition", "mgc_create_fixed_indegree_partition", "mgc_part_export", "mgc_part_import",
     "mgc_fault_inject_alloc", "mgc_selftest_wait_timeout", "mgc_partition_stats", "mgc_part_export_dev",
     "mgc_part_import_dev", "mgc_raster_stage", "mgc_raster_collect", "mgc_set_accumulation",
-    "mgc_create_generated", "mgc_gen_count",
+    "mgc_create_generated", "mgc_gen_count", "mgc_selftest_tile_timeout",
 )
 
 
@@ -163,6 +163,8 @@ def lib():
     for name in ("mgc_create_partition", "mgc_create_fixed_indegree_partition", "mgc_part_export",
                  "mgc_part_import", "mgc_fault_inject_alloc", "mgc_selftest_wait_timeout"):
         getattr(L, name).restype = C.c_int
+    L.mgc_selftest_tile_timeout.argtypes = [vp]
+    L.mgc_selftest_tile_timeout.restype = C.c_int
     L.mgc_run.argtypes = [vp, i64]
     L.mgc_sync.argtypes = [vp]
     L.mgc_set_rates.argtypes = [vp, vp, i32]
@@ -647,6 +649,11 @@ class Simulator:
         i = Info()
         check(lib().mgc_get_info(self._h, C.byref(i)))
         return {f: getattr(i, f) for f, _ in Info._fields_}
+
+    def selftest_tile_timeout(self):
+        """Lets the tiled step group's waits run out (no fault); sync() then
+        raises, until restore()."""
+        check(lib().mgc_selftest_tile_timeout(self._h))
 
     @property
     def kernel_launches(self):

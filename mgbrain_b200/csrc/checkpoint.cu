@@ -128,6 +128,9 @@ mgc_status mgc_checkpoint_load(mgc_sim* s, const void* buf, int64_t bytes)
         const int64_t none[2] = {0, -1};
         CK(cudaMemcpy(s->a.bits_span, none, sizeof(none), cudaMemcpyHostToDevice));
     }
+    // a wait that ran out since left its launch's counters behind
+    CKS(clear_tile_counters(s));
+    CK(cudaStreamSynchronize(s->stream));
     CK(cudaMemcpy(s->a.status, &zero32, 4, cudaMemcpyHostToDevice));
     if (s->a.ev_mark) {
         unsigned long long ev = 0;

@@ -315,9 +315,7 @@ mgc_status mgc_run(mgc_sim* s, int64_t steps)
             cudaError_t e;
             if (s->tile_on) {
                 CKS(refresh_tiles(s));
-                void* targs[] = {&ga, &s->tile, &n};
-                e = cudaLaunchCooperativeKernel((const void*)tile_kernel(s), dim3(s->tile.T), dim3(kTileThreads),
-                                                targs, s->tile_smem, s->stream);
+                e = launch_tiles(s, ga, n, s->tile.T);
                 if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
                     cudaGetLastError();  // not all resident here: the other step groups
                     s->tile_on = false;
@@ -325,7 +323,6 @@ mgc_status mgc_run(mgc_sim* s, int64_t steps)
                     CKS(set_acc_mask(s, wanted_acc_mask(s), true));
                     continue;
                 }
-                if (e == cudaSuccess) s->tile.epoch += (uint32_t)((n + s->tile.W - 1) / s->tile.W + 1);  // windows, the end
             } else if (p == 3) {
                 int32_t w = s->window;
                 // a window of w steps holds w buffers; each instantiation

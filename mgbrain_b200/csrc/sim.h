@@ -283,6 +283,10 @@ void release_in_rows(mgc_sim* s);
 mgc_status build_tiles(mgc_sim* s);
 // STDP: the tiles' weights brought up to date before they run (enqueued).
 mgc_status refresh_tiles(mgc_sim* s);
+// One launch of the tiled group: n steps, on `blocks` blocks (its tiles).
+cudaError_t launch_tiles(mgc_sim* s, StepArgs& a, int32_t n, int32_t blocks);
+// The step counters and a.done as a finished launch leaves them (enqueued).
+mgc_status clear_tile_counters(mgc_sim* s);
 // In-place exclusive scan of count + 1 entries (the last becomes the total).
 mgc_status scan_offsets(uint32_t* v, int64_t count, cudaStream_t st);
 // The readout's buffers (readout.cu).

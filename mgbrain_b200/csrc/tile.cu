@@ -2,6 +2,8 @@
 // by tile, and the kernel instantiations.
 #include "sim.h"
 
+using namespace mgc;
+
 namespace mgc {
 namespace {
 
@@ -370,6 +372,22 @@ mgc_status build_tiles(mgc_sim* s)
     return MGC_OK;
 }
 
+cudaError_t launch_tiles(mgc_sim* s, StepArgs& a, int32_t n, int32_t blocks)
+{
+    void* args[] = {&a, &s->tile, &n};
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void*)tile_kernel(s), dim3(blocks), dim3(kTileThreads),
+                                                      args, s->tile_smem, s->stream);
+    if (e == cudaSuccess) s->tile.epoch += (uint32_t)((n + s->tile.W - 1) / s->tile.W + 1);  // windows, the end
+    return e;
+}
+
+mgc_status clear_tile_counters(mgc_sim* s)
+{
+    if (s->tile.cnt) CK(cudaMemsetAsync(s->tile.cnt, 0, 4 * sizeof(int32_t) * kTileWindow * kTileLine, s->stream));
+    CK(cudaMemsetAsync(s->a.done, 0, sizeof(unsigned int), s->stream));
+    return MGC_OK;
+}
+
 mgc_status refresh_tiles(mgc_sim* s)
 {
     if (!s->tile_stale) return MGC_OK;
@@ -382,3 +400,16 @@ mgc_status refresh_tiles(mgc_sim* s)
 }
 
 }  // namespace mgc
+
+extern "C" mgc_status mgc_selftest_tile_timeout(mgc_sim* s)
+{
+    if (!s) return fail(MGC_ERR_INVALID, "null handle");
+    if (!s->tile_on || s->tile.T < 2) return fail(MGC_ERR_INVALID, "the handle's steps do not run on two or more tiles");
+    CK(cudaSetDevice(s->device));
+    CKS(refresh_tiles(s));
+    StepArgs a = s->a;
+    a.trace = nullptr;
+    CK(launch_tiles(s, a, 1, s->tile.T - 1));  // the last tile's block never publishes
+    s->launches += 1;
+    return MGC_OK;
+}

@@ -805,6 +805,14 @@ __device__ __forceinline__ bool tile_gather(const StepArgs& a, const TileArgs& t
     return *abort_flag == 0;
 }
 
+// After a wait that ran out, the step counters and a.done hold part of that
+// launch: places computed from them could lie outside the history.  No launch
+// runs any more until a checkpoint is loaded, which clears them and the status.
+__device__ __forceinline__ int tile_refused(const StepArgs& a)
+{
+    return (*(volatile int32_t*)a.status & kStatusBarrier) != 0;
+}
+
 template <bool CUR, bool FX, bool ONE>
 __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t, int32_t nsteps)
 {
@@ -860,12 +868,13 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
         if (tid < kTileWindow) scnt[tid] = 0;
         if (tid < 4 * kTileWindow) ctot[tid / kTileWindow][tid % kTileWindow] = 0;
         if (tid == 0) {
-            abort_flag = 0;
+            abort_flag = tile_refused(a);
             blk_ev = 0;
             count = npg = total = 0;
         }
     }
     __syncthreads();
+    if (abort_flag) return;
     for (int g = tid; g < t.nl / 4; g += blockDim.x) {
         bool p = false;
         for (int q = 0; q < 4; ++q) p |= m.type[4 * g + q] == kPOISSON;
@@ -1121,11 +1130,12 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_stdp(StepArgs a, TileA
     if (tid < kTileWindow) scnt[tid] = 0;
     if (tid < 4) ctot[tid] = 0;
     if (tid == 0) {
-        abort_flag = 0;
+        abort_flag = tile_refused(a);
         blk_ev = 0;
         count = npg = total = 0;
     }
     __syncthreads();
+    if (abort_flag) return;
     for (int g = tid; g < t.nl / 4; g += blockDim.x) {
         bool p = false;
         for (int x = 0; x < 4; ++x) p |= m.type[4 * g + x] == kPOISSON;

@@ -43,15 +43,16 @@ class Block:
 
 class Group:
     """One launch of `windows` windows over `tiles` blocks; load[k][b][w]: spikes
-    of warp w of block b in window k."""
+    of warp w of block b in window k; counter: what the step counters hold at its
+    start."""
 
-    def __init__(self, load, lists, seed):
+    def __init__(self, load, lists, seed, counter=0):
         self.load, self.lists = load, lists
         self.windows, self.tiles = len(load), len(load[0])
         self.rng = random.Random(seed)
         self.list = [[[] for _ in range(self.tiles)] for _ in range(lists)]
         self.mail = [[[(-1, 0, ())] * self.tiles for _ in range(self.tiles)] for _ in range(2)]  # [parity][reader][tile]
-        self.counter = [0] * SLOTS
+        self.counter = [counter] * SLOTS
         self.raster = [{} for _ in range(self.windows)]
         self.blocks = [Block(self.tiles) for _ in range(self.tiles)]
 
@@ -196,8 +197,10 @@ class Group:
         for k in range(self.windows):
             want = {self.spike(k, b, w, i) for b in range(self.tiles) for w in range(WARPS)
                     for i in range(self.load[k][b][w])}
-            if set(self.raster[k].values()) != want or len(self.raster[k]) != len(want):
+            if set(self.raster[k].values()) != want:
                 raise Failure(f"window {k}: raster {sorted(self.raster[k].values())}")
+            if sorted(self.raster[k]) != list(range(len(want))):
+                raise Failure(f"window {k}: places {sorted(self.raster[k])}")
         want = sorted(self.spike(k, b, w, i) for k in range(self.windows) for b in range(self.tiles)
                       for w in range(WARPS) for i in range(self.load[k][b][w]))
         for b, blk in enumerate(self.blocks):
@@ -231,3 +234,10 @@ def test_two_list_buffers_would_not_do():
         except Failure:
             failed += 1
     assert failed > 0
+
+
+def test_counters_must_be_zero_at_a_launch():
+    """A launch whose waits ran out leaves counts behind: the next one's raster
+    places would be off by them, and could lie past the history's end."""
+    with pytest.raises(Failure, match="places"):
+        Group([[[1, 1, 1]], [[1, 1, 1]]], kernel_lists(), 0, counter=5).run()
