@@ -64,8 +64,12 @@
 // Raster: a step's place in it needs the step's spikes of all tiles, so each
 // tile adds its counts to the window's 16 step counters when it publishes,
 // and writes its spikes' places one window later, when every tile's counts
-// are in: none of it is waited for.  The counters (slot k % 4) run on over the
-// windows of a launch; every block keeps their last totals.
+// are in: hardly ever waited for.  The counters (slot k % 4) run on over the
+// windows of a launch; every block keeps their last totals.  Nothing orders a
+// tile's additions before its next mailbox stores (both are relaxed), so a
+// reader reads the counters until the steps add up to the window's spikes, which
+// the mailboxes have told it; the first time while it waits for the next
+// window's mailboxes.
 //
 // Measured per step, the faster of the other step groups and this one: 4,000
 // neurons, minimum delay 1: 6.5 and 3.2 us; 11,000 neurons, windows of 15 steps
@@ -179,6 +183,23 @@ __device__ __forceinline__ TileSmem tile_smem(unsigned char* base, const TileArg
 __device__ __forceinline__ int32_t* tile_counter(const TileArgs& t, int k, int j)
 {
     return t.cnt + ((k & 3) * kTileWindow + j) * kTileLine;
+}
+__device__ __forceinline__ int32_t tile_count(const TileArgs& t, int k, int j)
+{
+    int32_t v;
+    asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(tile_counter(t, k, j)) : "memory");
+    return v;
+}
+// One more read of counters that did not add up; false: the limit is reached.
+__device__ __forceinline__ bool tile_again(const StepArgs& a, unsigned& it, int* late)
+{
+    if (++it > kBarrierSpins) {
+        atomicOr(a.status, kStatusBarrier);
+        *late = 1;
+        return false;
+    }
+    if (it > 64) __nanosleep(32);
+    return true;
 }
 
 // Network neuron of local neuron i of this block's tile.
@@ -817,7 +838,7 @@ template <bool CUR, bool FX, bool ONE>
 __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t, int32_t nsteps)
 {
     extern __shared__ __align__(16) unsigned char tile_raw[];
-    __shared__ int abort_flag;
+    __shared__ int abort_flag, late;  // waits that ran out: for the mailboxes, the counters
     __shared__ unsigned long long blk_ev;
     __shared__ int count, npg, total;  // the tile's spikes of the window, its POISSON groups, all tiles' spikes
     __shared__ uint32_t mine[kTileInline + 2];  // (a chunk's words past the last spike are read)
@@ -869,6 +890,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
         if (tid < 4 * kTileWindow) ctot[tid / kTileWindow][tid % kTileWindow] = 0;
         if (tid == 0) {
             abort_flag = tile_refused(a);
+            late = 0;
             blk_ev = 0;
             count = npg = total = 0;
         }
@@ -940,26 +962,28 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
         }
         rbase += stot[w];
     };
-    // running sums of window k's step totals, by the first warp
-    auto totals = [&](int k, int w) {
+    // running sums of window k's step totals (n_all in all), by the first warp;
+    // now: the counters as read before
+    auto totals = [&](int k, int w, int n_all, int32_t now) {
         if (tid < 32) {
-            int c = 0;
-            if (tid < w) {
-                const int32_t now = __ldcg(tile_counter(t, k, tid));
-                c = now - ctot[k & 3][tid];
-                ctot[k & 3][tid] = now;
-            }
+            int c;
+            for (unsigned it = 0;;) {
+                c = tid < w ? now - ctot[k & 3][tid] : 0;
 #pragma unroll
-            for (int o = 1; o < kTileWindow; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, c, o);
-                if (tid >= o) c += v;
+                for (int o = 1; o < kTileWindow; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, c, o);
+                    if (tid >= o) c += v;
+                }
+                if (__shfl_sync(0xffffffffu, c, kTileWindow - 1) == n_all || !tile_again(a, it, &late)) break;
+                if (tid < w) now = tile_count(t, k, tid);
             }
+            if (tid < w) ctot[k & 3][tid] = now;
             if (tid < w) stot[tid + 1] = c;
             if (tid == 0) stot[0] = 0;
         }
     };
     int slot = (int)(s0 % t.R);
-    int k = 0, c_prev = 0, w_prev = 0;  // the window before: this tile's spikes, steps
+    int k = 0, c_prev = 0, w_prev = 0, n_prev = 0;  // the window before: this tile's spikes, steps, all spikes
     int64_t w0 = s0;
     for (; w0 < s_end; ++k) {
         const int wl = (int)(s_end - w0 < t.W ? s_end - w0 : t.W);
@@ -972,6 +996,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
         int place = 0;
         if (tid >= 32 && tid < 32 + wl && scnt[tid - 32])
             place = atomicAdd(tile_counter(t, k, tid - 32), scnt[tid - 32]);
+        const int32_t early = k > 0 && tid < w_prev ? tile_count(t, k - 1, tid) : 0;
         const uint32_t* lists = t.list + (size_t)(k % kTileLists) * t.T * list_len;
         if (!tile_gather(a, t, m, k, lists, list_len, &total, &abort_flag)) return;
         if (tid >= 32 && tid < 32 + kTileWindow) {
@@ -979,14 +1004,16 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
             scnt[tid - 32] = 0;
         }
         if (tid == 0) count = 0;
-        if (k > 0) totals(k - 1, w_prev);
+        if (k > 0) totals(k - 1, w_prev, n_prev, early);
         TileSource src;
-        if (total <= kTileSpikes)
-            src.gathered(total);
+        n_prev = total;
+        if (n_prev <= kTileSpikes)
+            src.gathered(n_prev);
         else
             src.listed(TileSource::kTiles, t.T, k);
         tile_deliver<FX, ONE>(a, t, m, w0, slot, lo, hi, src, ev);
         __syncthreads();
+        if (late) return;
         if (tid == 0) total = 0;
         if (k > 0) record(k - 1, w0 - w_prev, w_prev, c_prev);
         c_prev = c_now;
@@ -998,8 +1025,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
     // the last window's raster and history: an empty window makes its counters final
     tile_publish(t, k, 0, mine);
     if (!tile_gather(a, t, m, k, t.list, 0, &total, &abort_flag)) return;
-    totals(k - 1, w_prev);
+    totals(k - 1, w_prev, n_prev, tid < w_prev ? tile_count(t, k - 1, tid) : 0);
     __syncthreads();
+    if (late) return;
     record(k - 1, w0 - w_prev, w_prev, c_prev);
     // back to the single-step form: the state, and the arrivals of s_end
 #pragma unroll 1
@@ -1078,7 +1106,7 @@ template <bool CUR>
 __global__ void __launch_bounds__(kTileThreads, 1) k_tile_stdp(StepArgs a, TileArgs t, int32_t nsteps)
 {
     extern __shared__ __align__(16) unsigned char tile_raw[];
-    __shared__ int abort_flag;
+    __shared__ int abort_flag, late;  // waits that ran out: for the mailboxes, the counters
     __shared__ unsigned long long blk_ev;
     __shared__ int count, npg, total;
     __shared__ uint32_t mine[kTileInline + 2];
@@ -1124,13 +1152,16 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_stdp(StepArgs a, TileA
             for (int h = 0; h < 2; ++h) ring[h * plane + row * t.stride + i] = in ? gring[h][from] : 0ull;
         }
     }
-    for (int i = tid; i < a.n; i += blockDim.x) q.lf[i] = a.last_fired[i];
+    // (a faster block may already have written a spike of step s0 here, which the
+    // exchange brings this block before anything reads it)
+    for (int i = tid; i < a.n; i += blockDim.x) q.lf[i] = __ldcg(a.last_fired + i);
     for (int i = tid; i < (a.n + 31) / 32; i += blockDim.x) q.fired[i] = 0;
     for (int i = tid; i <= t.nl; i += blockDim.x) q.in_off[i] = t.in_off[(size_t)tile * t.nl + i];
     if (tid < kTileWindow) scnt[tid] = 0;
     if (tid < 4) ctot[tid] = 0;
     if (tid == 0) {
         abort_flag = tile_refused(a);
+        late = 0;
         blk_ev = 0;
         count = npg = total = 0;
     }
@@ -1159,8 +1190,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_stdp(StepArgs a, TileA
                     f((int32_t)((m.cnt[l] > kTileInline ? __ldcg(tile_list(t, k, l) + x) : tile_mail(t, k, l, x)) & kTileId));
         }
     };
-    auto total_of = [&](int k) {  // step k's spikes (one thread, its counter final)
-        const int32_t now = __ldcg(tile_counter(t, k, 0));
+    // step k's spikes, n_all in all (one thread); now: the counter as read before
+    auto total_of = [&](int k, int n_all, int32_t now) {
+        for (unsigned it = 0; now - ctot[k & 3] != n_all && tile_again(a, it, &late);) now = tile_count(t, k, 0);
         stot = now - ctot[k & 3];
         ctot[k & 3] = now;
     };
@@ -1183,7 +1215,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_stdp(StepArgs a, TileA
         rbase += stot;
     };
     int slot = (int)(s0 % t.R);
-    int k = 0, c_prev = 0;
+    int k = 0, c_prev = 0, n_prev = 0;
     for (int64_t s = s0; s < s_end; ++s, ++k) {
         if (n_pg) tile_poisson(a, t, m, s, 1, n_pg, my_list(k), mine, &count, scnt);
         tile_update<CUR, true>(a, t, m, s, 1, slot, false, my_list(k), mine, &count, scnt);
@@ -1192,6 +1224,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_stdp(StepArgs a, TileA
         tile_publish(t, k, c_now, mine);
         int place = 0;
         if (tid == 32 && c_now) place = atomicAdd(tile_counter(t, k, 0), c_now);
+        const int32_t early = k > 0 && tid == 0 ? tile_count(t, k - 1, 0) : 0;
         if (!tile_gather(a, t, m, k, tile_list(t, k, 0), list_len, &total, &abort_flag)) return;
         if (tid == 32) {
             sbase[k & 1] = place - ctot[k & 3];
@@ -1199,14 +1232,16 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_stdp(StepArgs a, TileA
         }
         if (tid == 0) {
             count = 0;
-            if (k > 0) total_of(k - 1);
+            if (k > 0) total_of(k - 1, n_prev, early);
         }
+        n_prev = total;
         each_spike(k, tid, blockDim.x, [&](int32_t id) {
             if (!MGC_OK_INDEX(id >= 0 && id < a.n)) return;
             q.lf[id] = (int32_t)s;
             atomicOr(q.fired + (id >> 5), 1u << (id & 31));
         });
         __syncthreads();
+        if (late) return;
         // this tile's synapses of the spiking sources, eight lanes a source
         each_spike(k, tid >> 3, blockDim.x >> 3, [&](int32_t id) {
             if (!MGC_OK_INDEX(id >= 0 && id < a.n)) return;
@@ -1286,8 +1321,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_stdp(StepArgs a, TileA
     __syncthreads();
     tile_publish(t, k, 0, mine);
     if (!tile_gather(a, t, m, k, t.list, 0, &total, &abort_flag)) return;
-    if (tid == 0) total_of(k - 1);
+    if (tid == 0) total_of(k - 1, n_prev, tile_count(t, k - 1, 0));
     __syncthreads();
+    if (late) return;
     record(k - 1, s_end - 1, c_prev);
 #pragma unroll 1
     for (int i = tid; i < t.nl; i += blockDim.x) {

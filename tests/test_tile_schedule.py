@@ -1,6 +1,7 @@
 """The tiled step group's windows (k_tile), restated on the CPU: blocks of warps
 in random interleavings, with the kernel's list buffers, mailboxes, step counters
-and block barriers, and nothing else between them.  Every block must deliver each
+and block barriers, and nothing else between them; a counter's additions are seen
+by readers some time after they are made.  Every block must deliver each
 window's spikes exactly once, and every spike must get a raster place of its own
 in its own window.
 
@@ -44,15 +45,16 @@ class Block:
 class Group:
     """One launch of `windows` windows over `tiles` blocks; load[k][b][w]: spikes
     of warp w of block b in window k; counter: what the step counters hold at its
-    start."""
+    start; add_up: readers wait until a window's counts add up to its spikes."""
 
-    def __init__(self, load, lists, seed, counter=0):
-        self.load, self.lists = load, lists
+    def __init__(self, load, lists, seed, counter=0, add_up=True):
+        self.load, self.lists, self.add_up = load, lists, add_up
         self.windows, self.tiles = len(load), len(load[0])
         self.rng = random.Random(seed)
         self.list = [[[] for _ in range(self.tiles)] for _ in range(lists)]
         self.mail = [[[(-1, 0, ())] * self.tiles for _ in range(self.tiles)] for _ in range(2)]  # [parity][reader][tile]
         self.counter = [counter] * SLOTS
+        self.seen = list(self.counter)      # what a reader gets: the counters of some time ago
         self.raster = [{} for _ in range(self.windows)]
         self.blocks = [Block(self.tiles) for _ in range(self.tiles)]
 
@@ -87,8 +89,10 @@ class Group:
             self.raster[k][at] = e
             yield True
 
-    def totals(self, k, blk):
-        now = self.counter[k % SLOTS]
+    def totals(self, k, blk, n):
+        while self.add_up and self.seen[k % SLOTS] - blk.ctot[k % SLOTS] != n:
+            yield False
+        now = self.seen[k % SLOTS]
         blk.stot = now - blk.ctot[k % SLOTS]
         blk.ctot[k % SLOTS] = now
 
@@ -125,7 +129,7 @@ class Group:
 
     def warp(self, b, w):
         blk = self.blocks[b]
-        c_prev = 0
+        c_prev = n_prev = 0
         for k in range(self.windows):
             for i in range(self.load[k][b][w]):         # the update's spikes
                 pos = blk.count
@@ -152,7 +156,8 @@ class Group:
             if w == 0:
                 blk.count = 0
                 if k > 0:
-                    self.totals(k - 1, blk)
+                    yield from self.totals(k - 1, blk, n_prev)
+            n_prev = blk.total
             yield True
             if blk.total <= GATHERED:                    # the delivery
                 for q in range(w, blk.total, WARPS):
@@ -176,7 +181,7 @@ class Group:
             yield from self.publish(k, b, 0)
         yield from self.gather(k, b, w)
         if w == 0:
-            self.totals(k - 1, blk)
+            yield from self.totals(k - 1, blk, n_prev)
         yield from self.barrier(blk)
         yield from self.record(k - 1, b, w, c_prev)
 
@@ -187,6 +192,8 @@ class Group:
         while live:
             if self.rng.random() < 0.05:                 # some warps run ahead of the others for a while
                 weight = [self.rng.choice((1, 1, 30)) for _ in live]
+            if self.rng.random() < 0.02:
+                self.seen = list(self.counter)
             i = self.rng.choices(range(len(live)), weight[:len(live)])[0]
             try:
                 idle = 0 if next(live[i]) else idle + 1
@@ -240,4 +247,19 @@ def test_counters_must_be_zero_at_a_launch():
     """A launch whose waits ran out leaves counts behind: the next one's raster
     places would be off by them, and could lie past the history's end."""
     with pytest.raises(Failure, match="places"):
+        Group([[[1, 1, 1]], [[1, 1, 1]]], kernel_lists(), 0, counter=5, add_up=False).run()
+    with pytest.raises(Failure, match="waits"):
         Group([[[1, 1, 1]], [[1, 1, 1]]], kernel_lists(), 0, counter=5).run()
+
+
+def test_counters_are_read_until_they_add_up():
+    """The mailbox stores that tell of a window are not ordered after its counts."""
+    failed = 0
+    for seed in range(100):
+        try:
+            Group(loads(seed), kernel_lists(), seed, add_up=False).run()
+        except Failure:
+            failed += 1
+    assert failed > 0
+    for body in SOURCE.split("__global__")[1:]:      # both kernels read them so
+        assert re.search(r"n_all \|\| !tile_again\(|!= n_all && tile_again\(", body)
