@@ -332,6 +332,12 @@ mgc_status mgc_selftest_wait_timeout(int32_t device, int32_t which, int32_t* sta
  * two or more tiles.  No reference counterpart. */
 mgc_status mgc_selftest_tile_timeout(mgc_sim* sim);
 
+/* For tests of the tiled step group's window counter (32 bits, in every mailbox
+ * word): the next window counts as `epoch` (>= 1).  Results are the same.
+ * MGC_ERR_INVALID for a handle whose steps do not run in that group.  No reference
+ * counterpart. */
+mgc_status mgc_selftest_tile_epoch(mgc_sim* sim, uint32_t epoch);
+
 /* Enqueues `steps` steps on the handle's stream and returns without
  * waiting.  Replaces the step loop of MGSimulator::simulate_sparse
  * (mgsim.cpp:794-857) calling mgsim_step_sparse (mgcore.cu:535-554);

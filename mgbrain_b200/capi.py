@@ -38,6 +38,7 @@ EXPORTED = (
     "mgc_fault_inject_alloc", "mgc_selftest_wait_timeout", "mgc_partition_stats", "mgc_part_export_dev",
     "mgc_part_import_dev", "mgc_raster_stage", "mgc_raster_collect", "mgc_set_accumulation",
     "mgc_create_generated", "mgc_gen_count", "mgc_selftest_tile_timeout",
+    "mgc_selftest_tile_epoch",
 )
 
 
@@ -165,6 +166,8 @@ def lib():
         getattr(L, name).restype = C.c_int
     L.mgc_selftest_tile_timeout.argtypes = [vp]
     L.mgc_selftest_tile_timeout.restype = C.c_int
+    L.mgc_selftest_tile_epoch.argtypes = [vp, C.c_uint32]
+    L.mgc_selftest_tile_epoch.restype = C.c_int
     L.mgc_run.argtypes = [vp, i64]
     L.mgc_sync.argtypes = [vp]
     L.mgc_set_rates.argtypes = [vp, vp, i32]
@@ -654,6 +657,10 @@ class Simulator:
         """Lets the tiled step group's waits run out (no fault); sync() then
         raises, until restore()."""
         check(lib().mgc_selftest_tile_timeout(self._h))
+
+    def selftest_tile_epoch(self, epoch):
+        """The tiled step group's next window counts as `epoch`."""
+        check(lib().mgc_selftest_tile_epoch(self._h, int(epoch)))
 
     @property
     def kernel_launches(self):

@@ -372,12 +372,21 @@ mgc_status build_tiles(mgc_sim* s)
     return MGC_OK;
 }
 
+static size_t mail_bytes(const TileArgs& t) { return 2 * (size_t)t.T * t.T * kTileChunks * sizeof(ulonglong2); }
+
 cudaError_t launch_tiles(mgc_sim* s, StepArgs& a, int32_t n, int32_t blocks)
 {
+    const uint32_t windows = (uint32_t)((n + s->tile.W - 1) / s->tile.W + 1);  // and the end
+    if (s->tile.epoch > 0xffffffffu - windows) {
+        // epochs that wrapped would meet chunks last written 2^32 windows ago
+        const cudaError_t e = cudaMemsetAsync(s->tile.mail, 0, mail_bytes(s->tile), s->stream);
+        if (e != cudaSuccess) return e;
+        s->tile.epoch = 1;
+    }
     void* args[] = {&a, &s->tile, &n};
     const cudaError_t e = cudaLaunchCooperativeKernel((const void*)tile_kernel(s), dim3(blocks), dim3(kTileThreads),
                                                       args, s->tile_smem, s->stream);
-    if (e == cudaSuccess) s->tile.epoch += (uint32_t)((n + s->tile.W - 1) / s->tile.W + 1);  // windows, the end
+    if (e == cudaSuccess) s->tile.epoch += windows;
     return e;
 }
 
@@ -411,5 +420,15 @@ extern "C" mgc_status mgc_selftest_tile_timeout(mgc_sim* s)
     a.trace = nullptr;
     CK(launch_tiles(s, a, 1, s->tile.T - 1));  // the last tile's block never publishes
     s->launches += 1;
+    return MGC_OK;
+}
+
+extern "C" mgc_status mgc_selftest_tile_epoch(mgc_sim* s, uint32_t epoch)
+{
+    if (!s || epoch == 0) return fail(MGC_ERR_INVALID, "null handle, or epoch 0");
+    if (!s->tile_on) return fail(MGC_ERR_INVALID, "the handle's steps do not run on tiles");
+    CK(cudaSetDevice(s->device));
+    CK(cudaMemsetAsync(s->tile.mail, 0, mail_bytes(s->tile), s->stream));  // as if the epochs up to it had passed
+    s->tile.epoch = epoch;
     return MGC_OK;
 }

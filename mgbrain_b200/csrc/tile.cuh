@@ -106,7 +106,8 @@ struct TileArgs {
     const float* chain;   // [2][kTileTable] sums of k weights (exc, inh), when table
     uint32_t* list;       // [kTileLists][T][nl*W] spikes of a window: id | step in the window << 28
     ulonglong2* mail;     // [2][T reader][T][kTileChunks]
-    uint32_t epoch;       // epoch of the launch's first window (they count on over the launches)
+    uint32_t epoch;       // epoch of the launch's first window (they count on over the launches; never 0,
+                          //   which the mailboxes hold at first, and never past 2^32 - 1: launch_tiles)
     int32_t* cnt;         // [4][kTileWindow] counters (tile_counter) of a window's steps' spikes; zero between launches
     // plastic networks (k_tile_stdp): rec holds single records (off counts them)
     const uint32_t* cpos;   // [S] CSR position of a record

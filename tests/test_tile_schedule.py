@@ -19,7 +19,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 SOURCE = open(os.path.join(ROOT, "mgbrain_b200", "csrc", "tile.cuh")).read()
 
 WARPS = 3      # warp 0 publishes, polls and sums the counters; warp 1 reserves the places
-INLINE = 2     # spikes a mailbox place holds
+INLINE = 2     # spikes a mailbox place holds: one in its first chunk, one in its second
 GATHERED = 12  # spikes of a window that fit in shared memory
 SLOTS = 4      # counters
 
@@ -42,17 +42,23 @@ class Block:
         self.delivered = []     # per window
 
 
+def empty_mail(tiles):
+    """[parity][reader][tile] places of two chunks {epoch, count, spike}, {epoch, spike}, all zero."""
+    return [[[[(0, 0, None), (0, None)] for _ in range(tiles)] for _ in range(tiles)] for _ in range(2)]
+
+
 class Group:
     """One launch of `windows` windows over `tiles` blocks; load[k][b][w]: spikes
     of warp w of block b in window k; counter: what the step counters hold at its
-    start; add_up: readers wait until a window's counts add up to its spikes."""
+    start; add_up: readers wait until a window's counts add up to its spikes; mail,
+    epoch: what earlier launches left, the first window's epoch."""
 
-    def __init__(self, load, lists, seed, counter=0, add_up=True):
-        self.load, self.lists, self.add_up = load, lists, add_up
+    def __init__(self, load, lists, seed, counter=0, add_up=True, mail=None, epoch=1, epochs=1 << 32):
+        self.load, self.lists, self.add_up, self.epoch, self.epochs = load, lists, add_up, epoch, epochs
         self.windows, self.tiles = len(load), len(load[0])
         self.rng = random.Random(seed)
         self.list = [[[] for _ in range(self.tiles)] for _ in range(lists)]
-        self.mail = [[[(-1, 0, ())] * self.tiles for _ in range(self.tiles)] for _ in range(2)]  # [parity][reader][tile]
+        self.mail = mail or empty_mail(self.tiles)
         self.counter = [counter] * SLOTS
         self.seen = list(self.counter)      # what a reader gets: the counters of some time ago
         self.raster = [{} for _ in range(self.windows)]
@@ -102,9 +108,16 @@ class Group:
         if w == 0:
             blk.spikes = [None] * GATHERED
             for l in range(self.tiles):
-                while self.mail[k & 1][b][l][0] != k:
+                place = self.mail[k & 1][b][l]
+                epoch = (self.epoch + k) % self.epochs
+                while place[0][0] != epoch:
                     yield False
-                _, c, first = self.mail[k & 1][b][l]
+                _, c, e = place[0]
+                first = [e]
+                if 1 < c <= INLINE:
+                    while place[1][0] != epoch:
+                        yield False
+                    first.append(place[1][1])
                 at = blk.total
                 blk.total += c
                 blk.cnt[l] = (c, at)
@@ -123,9 +136,13 @@ class Group:
 
     def publish(self, k, b, c):
         blk = self.blocks[b]
+        epoch = (self.epoch + k) % self.epochs
         for r in range(self.tiles):
-            self.mail[k & 1][r][b] = (k, c, tuple(blk.mine))
+            self.mail[k & 1][r][b][0] = (epoch, c, blk.mine[0])
             yield True
+            if 1 < c <= INLINE:
+                self.mail[k & 1][r][b][1] = (epoch, blk.mine[1])
+                yield True
 
     def warp(self, b, w):
         blk = self.blocks[b]
@@ -168,7 +185,7 @@ class Group:
                     c, _ = blk.cnt[l]
                     for q in range(w, c, WARPS):
                         blk.delivered.append(self.list[k % self.lists][l][q] if c > INLINE
-                                             else self.mail[k & 1][b][l][2][q])
+                                             else self.mail[k & 1][b][l][q][-1])
                         yield True
             yield from self.barrier(blk)
             if w == 0:
@@ -211,7 +228,7 @@ class Group:
         want = sorted(self.spike(k, b, w, i) for k in range(self.windows) for b in range(self.tiles)
                       for w in range(WARPS) for i in range(self.load[k][b][w]))
         for b, blk in enumerate(self.blocks):
-            if sorted(blk.delivered) != want:
+            if None in blk.delivered or sorted(blk.delivered) != want:
                 raise Failure(f"tile {b} delivered other spikes")
 
 
@@ -263,3 +280,31 @@ def test_counters_are_read_until_they_add_up():
     assert failed > 0
     for body in SOURCE.split("__global__")[1:]:      # both kernels read them so
         assert re.search(r"n_all \|\| !tile_again\(|!= n_all && tile_again\(", body)
+
+
+def launches(seed, epochs, cleared):
+    """Launches on one handle whose epochs wrap; cleared: the mailboxes are, and the
+    epochs start again at 1, before a launch that would reach the wrap."""
+    rng = random.Random(seed)
+    tiles = rng.choice((2, 3))
+    mail, epoch = empty_mail(tiles), 1
+    for n in range(12):
+        load = [[[rng.choice((0, 0, 1)) for _ in range(WARPS)] for _ in range(tiles)]
+                for _ in range(rng.randint(1, 6))]
+        windows = len(load) + 1           # the last one is empty
+        if cleared and epoch + windows > epochs - 1:
+            mail, epoch = empty_mail(tiles), 1
+        Group(load, kernel_lists(), seed * 100 + n, mail=mail, epoch=epoch, epochs=epochs).run()
+        epoch += windows
+
+
+def test_epochs_that_wrap():
+    for seed in range(40):
+        launches(seed, 16, True)
+    failed = 0
+    for seed in range(40):
+        try:
+            launches(seed, 16, False)
+        except Failure:
+            failed += 1
+    assert failed > 0
