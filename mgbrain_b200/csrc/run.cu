@@ -318,7 +318,7 @@ mgc_status mgc_run(mgc_sim* s, int64_t steps)
                 e = launch_tiles(s, ga, n, s->tile.T);
                 if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
                     cudaGetLastError();  // not all resident here: the other step groups
-                    s->tile_on = false;
+                    s->tile_on = s->tile_wanted = false;
                     if (!s->a.deferred) break;
                     CKS(set_acc_mask(s, wanted_acc_mask(s), true));
                     continue;

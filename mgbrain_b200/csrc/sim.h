@@ -141,8 +141,9 @@ struct mgc_sim {
     int group_grid1 = 1;              // minimum delay 1: the step group's grid
     mgc::TileArgs tile{};             // tiled step group (tile.cuh): its layout, when the network
     bool tile_ok = false;             //   qualifies (build_tiles),
-    bool tile_on = false;             //   whether steps run in it (by default; an explicit step-group
-                                      //   mode or the autotuner may take another form)
+    bool tile_on = false;             //   whether steps run in it,
+    bool tile_wanted = true;          //   whether they should: until the caller or the autotuner
+                                      //   chooses another form
     bool tile_stale = false;          //   STDP: other forms changed the weights since its last step
     bool tile_one = false;            //   one delay, fp32 sums: 16-bit records
     size_t tile_smem = 0;             //   its dynamic shared memory

@@ -355,7 +355,8 @@ mgc_status build_tiles(mgc_sim* s)
         CK(cudaStreamSynchronize(s->stream));
         s->tile_smem = tile_stdp_bytes(t.nl, t.R, T, cur, s->n);
         CKS(allow_shared((const void*)tile_kernel(s), s->device));
-        s->tile_ok = s->tile_on = true;
+        s->tile_ok = true;
+        s->tile_on = s->tile_wanted;
         s->tile_stale = false;
         return MGC_OK;
     }
@@ -368,7 +369,8 @@ mgc_status build_tiles(mgc_sim* s)
     s->tile_one = one;
     s->tile_smem = tile_smem_bytes(t.nl, t.R, T, fx, cur, t.table != 0);
     CKS(allow_shared((const void*)tile_kernel(s), s->device));
-    s->tile_ok = s->tile_on = true;
+    s->tile_ok = true;
+    s->tile_on = s->tile_wanted;
     return MGC_OK;
 }
 

@@ -161,7 +161,7 @@ mgc_status mgc_set_persistent(mgc_sim* s, int32_t mode)
         s->sched_graph = false;
     }
     s->persistent = mode;
-    s->tile_on = s->auto_form = false;  // the caller's form, not the builder's choice
+    s->tile_on = s->tile_wanted = s->auto_form = false;  // the caller's form, not the builder's choice
     return MGC_OK;
 }
 
@@ -374,6 +374,7 @@ mgc_status mgc_autotune(mgc_sim* s, int64_t steps_per_trial, mgc_tune_report* re
         }
         if (st == MGC_OK) st = mgc_sync(s);
     }
+    s->tile_wanted = s->tile_on;
     s->persistent = rep->persistent;
     s->window = best_window;
     rep->window = s->fused ? s->window : 0;
