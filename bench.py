@@ -240,14 +240,23 @@ def cpu_baseline(w, sample_steps):
     return base, ref
 
 
-def parity_check(w, local, ref, steps, group_mode, window):
+def run_in(sim, form):
+    """The step form of another handle's step_form()."""
+    import mgbrain_b200 as mgb
+    if form["form"] == mgb.capi.FORM_TILED:
+        sim.set_tiled(True)
+        return
+    sim.set_persistent(form["form"])
+    if form["form"] == mgb.capi.FORM_WINDOWED:
+        sim.set_window(form["window"])
+
+
+def parity_check(w, local, ref, steps, form):
     """The GPU's first `steps` steps of the bench network, run from the same
     seeds in the step-group form the timed run used, against the oracle's."""
     sim = make_sim(w, local, seed=1, record=True)
     try:
-        sim.set_persistent(group_mode)
-        if group_mode == 3 and window:
-            sim.set_window(window)
+        run_in(sim, form)
         sim.run(steps)
         sim.sync()
         _, counts, ids = sim.read_raster(max_steps=steps + 1, max_ids=1 << 24)
@@ -260,7 +269,7 @@ def parity_check(w, local, ref, steps, group_mode, window):
     return {"steps": steps, "spikes": int(counts.sum()), "raster_equal": bool(raster_equal),
             "v_bit_equal": bool(np.array_equal(st["V"].view(np.int32), v_o.view(np.int32))),
             "v_max_rel": float(rel.max()), "fire_cnt_equal": bool(np.array_equal(st["fire_cnt"], ref["fire_cnt"])),
-            "step_group": {"mode": group_mode, "window": window},
+            "step_group": {"mode": form["form"], "window": form["window"] or None},
             "against": "oracle fp32 (C restatement of the reference kernels), same network and seeds"}
 
 
@@ -376,14 +385,14 @@ def run_ours(a, ws, rank, local):
         v["frac"] = v["achieved_gbs"] / hbm
         v["share"] = kms[0 if k_ == "neuron_update" else 1] / max(1e-9, sum(kms))
     steps_timed = a.steps * CHUNK
-    group_mode = sim.info()["persistent"]
-    sim_window = sim.info()["window"] if group_mode == 3 else None
-    if 0 < launches <= steps_timed and steps_timed % launches == 0:
+    form = sim.step_form()
+    group_mode, sim_window = form["form"], form["window"] or None
+    if 0 < launches <= steps_timed and (group_mode == 4 or steps_timed % launches == 0):
         # the fused method: one kernel per step (k_fused) or one per step group
-        # (k_steps / k_pipe / k_window); each launch covers steps_timed /
+        # (k_steps / k_pipe / k_window / k_tile); each launch covers steps_timed /
         # launches steps and its average duration is the timed region over its launches
-        per_launch = steps_timed // launches
-        dom = {0: "k_fused", 1: "k_steps", 2: "k_pipe", 3: "k_window"}[group_mode]
+        per_launch = steps_timed / launches
+        dom = {0: "k_fused", 1: "k_steps", 2: "k_pipe", 3: "k_window", 4: "k_tile"}[group_mode]
         dur_us = 1e3 * ms / launches
         dbytes = per_launch * (neuron_bytes + 8.0 * events / steps_timed)
         achieved = dbytes / (dur_us * 1e-6) / 1e9
@@ -479,7 +488,7 @@ def run_ours(a, ws, rank, local):
         fms, fev, _ = timed_device(simf, CHUNK, 1, ws)
         fms, fev = allmax(ws, fms), allsum(ws, fev)
         driven["fixed_point"] = {"events_per_s": fev / (fms / 1e3), "sim_s_per_wall_s": CHUNK * DT / (fms / 1e3),
-                                 "step_group": simf.info()["persistent"], "fx_shift": simf.info()["fx_shift"]}
+                                 "step_group": simf.step_form()["form"], "fx_shift": simf.info()["fx_shift"]}
         simf.close()
 
     pull = None
@@ -497,7 +506,7 @@ def run_ours(a, ws, rank, local):
             cpu, ref = {"value": None, "unit": "events/s", "cores": 1, "kind": "port",
                         "sample": f"not run: {e}"}, None
         if ref is not None:
-            parity = parity_check(w, local, ref, a.cpu_sample, group_mode, sim_window)
+            parity = parity_check(w, local, ref, a.cpu_sample, form)
     reference_gpu = None
     if rank == 0 and not a.no_refgpu:
         try:
@@ -551,8 +560,8 @@ def pull_variant(local, steps=3000, warm=1000):
         sim = brunel.burst_simulator(net, device=local, raster_ids=-1)
         if tune:
             t = sim.autotune(steps_per_trial=640)
-            form = {"persistent": t["persistent"], "window": t["window"], "chunk_len": t["chunk_len"],
-                    "pull_min_pairs": t["pull_min"]}
+            form = {"step_form": sim.step_form(), "persistent": t["persistent"], "window": t["window"],
+                    "chunk_len": t["chunk_len"], "pull_min_pairs": t["pull_min"]}
         else:
             sim.set_persistent(3)
             sim.set_window(8)

@@ -124,8 +124,8 @@ typedef struct mgc_info {
     int32_t mode;
     int32_t graph_steps;       /* steps per captured CUDA graph */
     int64_t device_bytes;      /* device memory held by the handle */
-    int32_t persistent;        /* steps run as step groups: 0 no (graphs), 1 barrier per step, 2 pipelined,
-                                  3 windowed */
+    int32_t persistent;        /* step-group mode (mgc_set_persistent): 0 none (graphs), 1 barrier per step,
+                                  2 pipelined, 3 windowed; mgc_get_step_form tells what runs in its place */
     int32_t first_neuron;      /* partition handles: whole-network id of neuron 0 (else 0) */
     int32_t total_neurons;     /* partition handles: neurons of the whole network (else n_neurons) */
     int32_t window;            /* steps per window of the windowed step group (0: minimum delay 1) */
@@ -414,10 +414,11 @@ typedef struct mgc_tune_report {
     int32_t chunk_len;            /* chosen synapses per delivery task (deferred method) */
     int32_t blocks_per_sm;        /* chosen resident blocks per SM of the step's main kernel (0: the
                                      ring or pull method's push on fewer blocks than SMs) */
-    int32_t persistent;           /* chosen step-group mode of the fused method (mgc_set_persistent) */
+    int32_t persistent;           /* chosen step-group mode of the fused method (mgc_set_persistent): the
+                                     fastest but for the tiled group, which mgc_get_step_form tells of */
     int32_t window;               /* chosen window of the windowed step group (mgc_set_window) */
     int32_t pull_min;             /* chosen pull-step threshold (mgc_set_pull), 0: none */
-    double ms_per_step;           /* time per step of the chosen configuration */
+    double ms_per_step;           /* time per step of the chosen configuration (the tiled group's, if it runs) */
     double default_ms_per_step;   /* time per step of the builder's configuration */
     int64_t steps;                /* steps simulated by the trials */
 } mgc_tune_report;
@@ -458,18 +459,37 @@ mgc_status mgc_autotune_rewind(mgc_sim* sim, int64_t steps_per_trial, mgc_tune_r
  * windowed step groups (minimum delay >= 2): the arrivals of a window of W
  * steps (mgc_set_window) are delivered before it, then every neuron advances
  * the W steps with its state in registers, two grid barriers per window.
- * Default: 2 when the minimum delay is >= 4, else 1; the autotuner may pick
- * another.  By default, and when the autotuner finds it fastest, a network
- * whose state fits on the chip runs the tiled step group in the place of that
- * mode (one block per SM keeps its neurons' state and inputs in shared memory
- * and delivers every spike to its own targets from a copy of the synapses cut
- * by block), and other networks run the windowed group in the place of mode 2;
- * a mode set here runs as described.  If the device cannot keep all blocks of a group resident, the
+ * Until a mode is set here or by the autotuner, the mode is 2 when the minimum
+ * delay is >= 4, else 1, and a faster form of the same results runs in its place
+ * where there is one: the tiled group (mgc_set_tiled), else the windowed group in
+ * the place of 2.  A mode set here runs as described.  If the device cannot keep all blocks of a group resident, the
  * call falls back to 0.  Results are the same in every mode; while a schedule mode other than
  * static, recording or calibration is on, graphs are used.  All waits are
  * bounded (a time-out makes mgc_sync return MGC_ERR_CUDA).  No reference
  * counterpart. */
 mgc_status mgc_set_persistent(mgc_sim* sim, int32_t mode);
+
+/* The tiled step group: one block per SM keeps its neurons' state and inputs in
+ * shared memory and delivers every spike to its own targets from a copy of the
+ * synapses cut by block.  A network whose state fits on the chip runs in it until
+ * mgc_set_persistent or the autotuner chooses another form.  on != 0: steps run
+ * in it again (MGC_ERR_INVALID for a network that has no such layout); 0: in the
+ * mode of mgc_set_persistent, or in the form that runs in its place.  Results are
+ * the same.  No reference counterpart. */
+mgc_status mgc_set_tiled(mgc_sim* sim, int32_t on);
+
+/* The form in which the next mgc_run's steps run. */
+enum { MGC_FORM_GRAPHS = 0, MGC_FORM_BARRIER = 1, MGC_FORM_PIPELINED = 2, MGC_FORM_WINDOWED = 3,
+       MGC_FORM_TILED = 4 };
+
+typedef struct mgc_step_form {
+    int32_t form;              /* MGC_FORM_*; GRAPHS for methods without step groups too */
+    int32_t window;            /* WINDOWED, TILED: steps per window (else 0) */
+    int32_t tiles;             /* TILED: blocks (else 0) */
+    int32_t tile_neurons;      /* TILED: neurons of a block, in groups of four dealt to the blocks in turn */
+} mgc_step_form;
+
+mgc_status mgc_get_step_form(mgc_sim* sim, mgc_step_form* form);
 
 /* Pull steps (deferred method, minimum delay >= 2, not for partition
  * handles): in the windowed step group (mgc_set_persistent mode 3), a step

@@ -23,6 +23,7 @@ RAW, LIF0, POISSON, LIF, LIFE, LIFB = range(6)
 MODE_AUTO, MODE_PUSH, MODE_DEFERRED, MODE_PULL = 0, 1, 2, 3
 SCHED_STATIC, SCHED_THRESHOLD, SCHED_LEARNED = 0, 1, 2
 ACC_FLOAT, ACC_FIXED = 0, 1
+FORM_GRAPHS, FORM_BARRIER, FORM_PIPELINED, FORM_WINDOWED, FORM_TILED = range(5)
 RULE_PROB, RULE_ALL, RULE_ONE, RULE_ALL_BUT_SELF, RULE_FIXED_INDEGREE = range(5)
 MLP_IN, MLP_HIDDEN, MLP_OUT, MLP_PARAMS = 20, 32, 5, 837
 
@@ -38,7 +39,7 @@ EXPORTED = (
     "mgc_fault_inject_alloc", "mgc_selftest_wait_timeout", "mgc_partition_stats", "mgc_part_export_dev",
     "mgc_part_import_dev", "mgc_raster_stage", "mgc_raster_collect", "mgc_set_accumulation",
     "mgc_create_generated", "mgc_gen_count", "mgc_selftest_tile_timeout",
-    "mgc_selftest_tile_epoch",
+    "mgc_selftest_tile_epoch", "mgc_set_tiled", "mgc_get_step_form",
 )
 
 
@@ -128,6 +129,10 @@ class Info(C.Structure):
     ]
 
 
+class StepForm(C.Structure):
+    _fields_ = [("form", C.c_int32), ("window", C.c_int32), ("tiles", C.c_int32), ("tile_neurons", C.c_int32)]
+
+
 _lib = None
 
 
@@ -195,6 +200,10 @@ def lib():
     L.mgc_autotune_rewind.restype = C.c_int
     L.mgc_set_persistent.argtypes = [vp, i32]
     L.mgc_set_persistent.restype = C.c_int
+    L.mgc_set_tiled.argtypes = [vp, i32]
+    L.mgc_set_tiled.restype = C.c_int
+    L.mgc_get_step_form.argtypes = [vp, C.POINTER(StepForm)]
+    L.mgc_get_step_form.restype = C.c_int
     L.mgc_set_pull.argtypes = [vp, i32]
     L.mgc_set_pull.restype = C.c_int
     L.mgc_set_window.argtypes = [vp, i32]
@@ -624,6 +633,18 @@ class Simulator:
         with a grid barrier per step; 2: pipelined step groups; 3: windowed
         step groups (set_window)."""
         check(lib().mgc_set_persistent(self._h, int(mode)))
+
+    def set_tiled(self, on=True):
+        """Steps run in the tiled step group (which networks whose state fits on
+        the chip start in), or, with False, in the mode of set_persistent."""
+        check(lib().mgc_set_tiled(self._h, int(bool(on))))
+
+    def step_form(self):
+        """The form in which the next steps run: form (one of FORM_*), window,
+        tiles, tile_neurons (mgc_get_step_form)."""
+        f = StepForm()
+        check(lib().mgc_get_step_form(self._h, C.byref(f)))
+        return {k: getattr(f, k) for k, _ in StepForm._fields_}
 
     def set_accumulation(self, mode):
         """ACC_FLOAT (fp32 additions) or ACC_FIXED (order-independent 64-bit

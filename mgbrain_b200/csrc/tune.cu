@@ -165,6 +165,28 @@ mgc_status mgc_set_persistent(mgc_sim* s, int32_t mode)
     return MGC_OK;
 }
 
+mgc_status mgc_set_tiled(mgc_sim* s, int32_t on)
+{
+    if (!s) return fail(MGC_ERR_INVALID, "null handle");
+    if (on && !s->tile_ok) return fail(MGC_ERR_INVALID, "the network has no layout for the tiled step group");
+    s->tile_on = s->tile_wanted = on != 0;
+    return MGC_OK;
+}
+
+mgc_status mgc_get_step_form(mgc_sim* s, mgc_step_form* f)
+{
+    if (!s || !f) return fail(MGC_ERR_INVALID, "null argument");
+    *f = mgc_step_form{MGC_FORM_GRAPHS, 0, 0, 0};
+    if (sched_wanted(s)) return MGC_OK;
+    if (s->tile_on) {
+        *f = mgc_step_form{MGC_FORM_TILED, s->tile.W, s->tile.T, s->tile.nl};
+    } else if (s->a.deferred) {
+        f->form = group_mode(s);
+        f->window = f->form == MGC_FORM_WINDOWED ? s->window : 0;
+    }
+    return MGC_OK;
+}
+
 mgc_status mgc_set_pull(mgc_sim* s, int32_t min_pairs)
 {
     if (!s) return fail(MGC_ERR_INVALID, "null handle");
@@ -348,10 +370,9 @@ mgc_status mgc_autotune(mgc_sim* s, int64_t steps_per_trial, mgc_tune_report* re
         if (st == MGC_OK) st = mgc_sync(s);
     }
     if (pull_ok && st == MGC_OK) st = mgc_set_pull(s, 0);
-    // the tiled step group, where the network has its layout: it runs in the
-    // place of the builder's default step-group mode
+    // the tiled step group, where the network has its layout: the report keeps
+    // the fastest of the other forms, which runs when the tiles are turned off
     if (s->tile_ok && st == MGC_OK && !sched_wanted(s)) {
-        s->persistent = !s->a.deferred ? 0 : (s->dmin >= 4 ? 2 : 1);
         s->tile_on = true;
         st = mgc_run(s, kGraphSteps);
         if (st == MGC_OK) {
@@ -363,14 +384,10 @@ mgc_status mgc_autotune(mgc_sim* s, int64_t steps_per_trial, mgc_tune_report* re
         if (st == MGC_OK && cudaEventSynchronize(e1) == cudaSuccess && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess) {
             const double per = (double)ms / (double)steps;
             rep->trials += 1;
-            if (per < best && s->tile_on) {
+            if (per < best && s->tile_on)
                 best = per;
-                rep->persistent = s->persistent;
-                best_window = window0;
-                best_pull = 0;
-            } else {
+            else
                 s->tile_on = false;
-            }
         }
         if (st == MGC_OK) st = mgc_sync(s);
     }
@@ -382,7 +399,7 @@ mgc_status mgc_autotune(mgc_sim* s, int64_t steps_per_trial, mgc_tune_report* re
     cudaEventDestroy(e1);
     if (st != MGC_OK) return st;
     CKS(apply_cand(s, best_c, sms));
-    if (best_pull > 0)
+    if (best_pull > 0 && !s->tile_on)
         CKS(mgc_set_pull(s, best_pull));
     else if (pull_ok && !had_rows)
         release_in_rows(s);  // the trials' incoming rows, not needed
