@@ -312,7 +312,8 @@ mgc_status mgc_part_import_dev(mgc_sim* sim, int32_t count, int32_t nranks, int3
 /* Host-side fault injection for callers' error paths: the n-th device
  * allocation from now (n >= 1) fails as if the device were out of memory;
  * 0 turns it off.  The entry point that meets it returns MGC_ERR_NOMEM and
- * frees what it had allocated.  No reference counterpart (the reference's
+ * frees what it had allocated, or does without the memory where it can (the
+ * tiled group's layout, buffers that only save time).  No reference counterpart (the reference's
  * CUDACHECK exits the process, cudamem.cuh:8-18). */
 mgc_status mgc_fault_inject_alloc(int64_t n);
 

@@ -560,8 +560,8 @@ mgc_status finish_build(mgc_sim* s)
     }
     a.M = s->M;
     CKS(launch_shapes(s));
-    CKS(build_tiles(s));
     CKS(init_readout(s));
+    CKS(build_tiles(s));  // (last: whatever else the handle needs has its memory)
     CK(cudaStreamSynchronize(s->stream));
     return MGC_OK;
 }

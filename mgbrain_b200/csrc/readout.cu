@@ -240,15 +240,11 @@ constexpr int32_t kStateOneCopy = 1 << 16;
 
 namespace mgc {
 
-mgc_status init_readout(mgc_sim* s)
+// The raster's sort: its sums, its launch shape, and bitmaps for networks whose
+// ids' bitmap does not fit in shared memory (fewer of them, each for a block,
+// where the device has no room for all).
+static mgc_status init_raster(mgc_sim* s)
 {
-    if (s->n <= kStateOneCopy) {
-        CKS(s->alloc(&s->state_buf, 6 * (size_t)s->n, false));
-        s->state_host.resize(6 * (size_t)s->n);
-    }
-    // weights that change are read again and again (cudaMalloc and cudaFree in
-    // the call took up to 600 ms on a busy driver)
-    if (s->stdp && s->S > 0) CKS(s->alloc(&s->weights_buf, s->S, false));
     if (!s->a.record) return MGC_OK;
     CKS(s->alloc(&s->raster_meta, 5));
     CKS(s->alloc(&s->raster_off, (size_t)s->raster_steps_cap + 1, false));
@@ -262,9 +258,28 @@ mgc_status init_readout(mgc_sim* s)
     s->sort_grid = sms * std::max(1, occ);
     if (!chip) {
         s->sort_grid = (int)std::max<int64_t>(1, std::min<int64_t>(sms, kSortBitmaps / (4 * s->sort_words)));
-        CKS(s->alloc(&s->sort_bitmap, (size_t)s->sort_grid * (size_t)s->sort_words, false));
+        for (;; s->sort_grid /= 2) {
+            const mgc_status st = s->alloc(&s->sort_bitmap, (size_t)s->sort_grid * (size_t)s->sort_words, false);
+            if (st == MGC_OK) break;
+            if (st != MGC_ERR_NOMEM || s->sort_grid == 1) return st;
+        }
     }
     return MGC_OK;
+}
+
+mgc_status init_readout(mgc_sim* s)
+{
+    if (s->n <= kStateOneCopy) {
+        CKS(s->alloc(&s->state_buf, 6 * (size_t)s->n, false));
+        s->state_host.resize(6 * (size_t)s->n);
+    }
+    CKS(init_raster(s));
+    // weights that change are read again and again (cudaMalloc and cudaFree in
+    // the call took up to 600 ms on a busy driver); without the buffer, each
+    // call finds its own
+    if (!s->stdp || s->S == 0) return MGC_OK;
+    const mgc_status st = s->alloc(&s->weights_buf, s->S, false);
+    return st == MGC_ERR_NOMEM ? MGC_OK : st;
 }
 
 }  // namespace mgc

@@ -280,7 +280,8 @@ mgc_status build_in_rows(mgc_sim* s);
 // Frees them again (pull steps off; the stream idle first).
 void release_in_rows(mgc_sim* s);
 // The tiled step group's synapses and buffers, when the network qualifies for
-// it (tile.cu); built again when the accumulation changes.
+// it and they fit in the device's memory (tile.cu); built again when the
+// accumulation changes.
 mgc_status build_tiles(mgc_sim* s);
 // STDP: the tiles' weights brought up to date before they run (enqueued).
 mgc_status refresh_tiles(mgc_sim* s);

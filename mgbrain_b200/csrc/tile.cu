@@ -226,10 +226,9 @@ void release_tiles(mgc_sim* s)
     s->tile_ok = s->tile_on = false;
 }
 
-mgc_status build_tiles(mgc_sim* s)
+static mgc_status lay_tiles(mgc_sim* s)
 {
     StepArgs& a = s->a;
-    release_tiles(s);
     const bool stdp = s->stdp && !a.deferred && !a.pull && a.fx;  // the ring method with STDP
     if ((!a.deferred && !stdp) || s->partition || s->S <= 0 || (s->hetero && !a.fx) || s->dmax > kTileMaxDelay)
         return MGC_OK;
@@ -375,6 +374,16 @@ mgc_status build_tiles(mgc_sim* s)
 }
 
 static size_t mail_bytes(const TileArgs& t) { return 2 * (size_t)t.T * t.T * kTileChunks * sizeof(ulonglong2); }
+
+mgc_status build_tiles(mgc_sim* s)
+{
+    release_tiles(s);
+    const mgc_status st = lay_tiles(s);
+    if (st == MGC_OK) return st;
+    cudaStreamSynchronize(s->stream);
+    release_tiles(s);
+    return st == MGC_ERR_NOMEM ? MGC_OK : st;  // the network runs without them
+}
 
 cudaError_t launch_tiles(mgc_sim* s, StepArgs& a, int32_t n, int32_t blocks)
 {

@@ -1,0 +1,66 @@
+"""Device memory that only makes a handle faster (the tiled group's copy of the
+synapses, the kept buffer of plastic weights) is done without where the device has
+none: the network is built and runs in another form, with the same results."""
+import gc
+
+import numpy as np
+import pytest
+import torch
+
+import mgbrain_b200 as mgb
+import test_tile_group_gpu as group
+import test_tile_stdp_gpu as plastic
+from mgbrain_b200 import capi
+
+NETS = {"one_delay": (group.network, group.CASES["one_delay"][0]),
+        "ranged": (group.network, group.CASES["ranged"][0]),
+        "plastic": (plastic.network, plastic.CASES["delays"])}
+
+
+def outcome(sim):
+    sim.run(300)
+    sim.sync()
+    return sim.read_raster(), sim.state(), sim.weights()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", sorted(NETS))
+def test_networks_are_built_without_the_tiles_memory(name):
+    build, spec = NETS[name]
+    args, kw = build(seed=7, **spec)
+    make = lambda: mgb.Simulator.from_arrays(*args, **dict(kw, seed=5))  # noqa: E731
+    ref = make()
+    ref.set_persistent(0)
+    want = outcome(ref)
+    ref.close()
+    gc.collect()
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    without = k = 0
+    while True:
+        k += 1
+        assert k < 500
+        mgb.fault_inject_alloc(k)
+        try:
+            sim = make()
+        except mgb.MgcError as e:
+            assert e.status == capi.MGC_ERR_NOMEM and without == 0, (k, str(e))
+            continue                          # memory that the handle cannot do without
+        finally:
+            mgb.fault_inject_alloc(0)
+        tiled = sim.step_form()["form"] == capi.FORM_TILED
+        if not tiled or without == 0:
+            got = outcome(sim)
+            for x, y in zip(want[0], got[0]):
+                assert np.array_equal(x, y)
+            for key in want[1]:
+                assert np.array_equal(want[1][key].view(np.int32), got[1][key].view(np.int32)), key
+            assert np.array_equal(want[2].view(np.int32), got[2].view(np.int32))
+        sim.close()
+        without += not tiled
+        if tiled and without > 0:
+            break
+    assert without >= 6                       # several of its allocations, each given up cleanly
+    gc.collect()
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] > free0 - (64 << 20)
