@@ -917,15 +917,25 @@ mgc_status build_in_rows(mgc_sim* s)
     if (a.in_ent) return MGC_OK;
     const int64_t S = s->S;
     if (S >= (int64_t(1) << 32)) return fail(MGC_ERR_INVALID, "pull steps need fewer than 2^32 synapses");
-    int64_t* in_ptr = nullptr;
+    int64_t *in_ptr = nullptr, *span = nullptr;
     uint2* in_ent = nullptr;
     uint32_t* bits = nullptr;
+    struct Guard {  // frees what was allocated when a later step fails
+        mgc_sim* s;
+        void* const rows[4];
+        ~Guard()
+        {
+            if (s->a.in_ent) return;
+            cudaStreamSynchronize(s->stream);
+            for (void* p : rows)
+                if (*static_cast<void**>(p)) s->release(*static_cast<void**>(p));
+        }
+    } guard{s, {&in_ptr, &in_ent, &bits, &span}};
     const int64_t groups = a.ns / 4;
     const int32_t words = (int32_t)((groups + 31) / 32 * 4);
     CKS(s->alloc(&in_ptr, (size_t)s->n + 1));
     CKS(s->alloc(&in_ent, (size_t)std::max<int64_t>(S, 1), false));
     CKS(s->alloc(&bits, (size_t)a.H * (size_t)words));
-    int64_t* span = nullptr;
     CKS(s->alloc(&span, 2));
     {
         DevTmp t_k, t_k2, t_p, t_o, t_s;
@@ -947,13 +957,13 @@ mgc_status build_in_rows(mgc_sim* s)
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(s->stream));
     }
+    const int64_t none[2] = {0, -1};  // no step has its bitmap yet
+    CK(cudaMemcpy(span, none, sizeof(none), cudaMemcpyHostToDevice));
     a.in_ptr = in_ptr;
     a.in_ent = in_ent;
     a.hist_bits = bits;
     a.bits_words = words;
     a.bits_span = span;
-    const int64_t none[2] = {0, -1};  // no step has its bitmap yet
-    CK(cudaMemcpy(span, none, sizeof(none), cudaMemcpyHostToDevice));
     return MGC_OK;
 }
 
@@ -1310,7 +1320,7 @@ extern "C" mgc_status mgc_set_accumulation(mgc_sim* s, int32_t mode)
     }
     a.fx = fx;
     CKS(launch_shapes(s));
-    CKS(build_tiles(s));
+    if (s->tile_wanted) CKS(build_tiles(s));
     CK(cudaStreamSynchronize(s->stream));
     return MGC_OK;
 }

@@ -318,7 +318,8 @@ mgc_status mgc_run(mgc_sim* s, int64_t steps)
                 e = launch_tiles(s, ga, n, s->tile.T);
                 if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
                     cudaGetLastError();  // not all resident here: the other step groups
-                    s->tile_on = s->tile_wanted = false;
+                    s->tile_wanted = false;
+                    drop_tiles(s);
                     if (!s->a.deferred) break;
                     CKS(set_acc_mask(s, wanted_acc_mask(s), true));
                     continue;

@@ -71,6 +71,11 @@ inline int grid_for(int64_t n, int block = 256)
 
 }  // namespace mgc
 
+namespace mgc {
+// Waits for the stream and frees the tiled step group's layout (tile.cu).
+void drop_tiles(mgc_sim* s);
+}  // namespace mgc
+
 struct mgc_sim {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -140,7 +145,7 @@ struct mgc_sim {
     int acc_buffers = 4;              // accumulator buffers allocated (8 for a minimum delay >= 5)
     int group_grid1 = 1;              // minimum delay 1: the step group's grid
     mgc::TileArgs tile{};             // tiled step group (tile.cuh): its layout, when the network
-    bool tile_ok = false;             //   qualifies (build_tiles),
+    bool tile_ok = false;             //   qualifies and holds it (build_tiles),
     bool tile_on = false;             //   whether steps run in it,
     bool tile_wanted = true;          //   whether they should: until the caller or the autotuner
                                       //   chooses another form
@@ -169,7 +174,13 @@ struct mgc_sim {
     {
         void* v = nullptr;
         size_t b = std::max<size_t>(count, 1) * sizeof(T);
-        CK(mgc::dev_malloc(&v, b));
+        cudaError_t e = mgc::dev_malloc(&v, b);
+        if (e == cudaErrorMemoryAllocation && tile_ok) {  // what the handle must have comes before the tiles
+            cudaGetLastError();
+            mgc::drop_tiles(this);
+            e = mgc::dev_malloc(&v, b);
+        }
+        CK(e);
         allocs.push_back(v);
         alloc_bytes.push_back(b);
         bytes += b;

@@ -215,8 +215,9 @@ TileKernel tile_kernel(const mgc_sim* s)
     return s->tile_one ? tile_of<false, true>(s->a.has_cur) : tile_of<false, false>(s->a.has_cur);
 }
 
-void release_tiles(mgc_sim* s)
+void drop_tiles(mgc_sim* s)
 {
+    cudaStreamSynchronize(s->stream);
     TileArgs& t = s->tile;
     for (const void* p : {(const void*)t.off, t.rec, (const void*)t.we, (const void*)t.wi, (const void*)t.chain,
                           (const void*)t.list, (const void*)t.mail, (const void*)t.cnt, (const void*)t.cpos,
@@ -260,7 +261,8 @@ static mgc_status lay_tiles(mgc_sim* s)
     if ((int64_t)s->n * T + 1 > (int64_t)0x7fffffff || most / vec_bytes > kIndex / 2) return MGC_OK;
     size_t free_b = 0, total_b = 0;
     CK(cudaMemGetInfo(&free_b, &total_b));
-    if (need > free_b / 2) return MGC_OK;
+    // the copy only saves time: it leaves seven eighths of what is free to others
+    if (need > free_b / 8) return MGC_OK;
     TileArgs& t = s->tile;
     t.T = T;
     t.nl = (int32_t)nl_of(T);
@@ -316,7 +318,7 @@ static mgc_status lay_tiles(mgc_sim* s)
     }
     if (!fx) {
         if (h[4] > 0xffffu) {  // a step's count of one sign might not fit its half word
-            release_tiles(s);
+            drop_tiles(s);
             return MGC_OK;
         }
         t.table = (h[0] >= h[1] && h[2] >= h[3]) ? 1 : 0;
@@ -377,11 +379,10 @@ static size_t mail_bytes(const TileArgs& t) { return 2 * (size_t)t.T * t.T * kTi
 
 mgc_status build_tiles(mgc_sim* s)
 {
-    release_tiles(s);
+    drop_tiles(s);
     const mgc_status st = lay_tiles(s);
     if (st == MGC_OK) return st;
-    cudaStreamSynchronize(s->stream);
-    release_tiles(s);
+    drop_tiles(s);
     return st == MGC_ERR_NOMEM ? MGC_OK : st;  // the network runs without them
 }
 

@@ -161,16 +161,27 @@ mgc_status mgc_set_persistent(mgc_sim* s, int32_t mode)
         s->sched_graph = false;
     }
     s->persistent = mode;
-    s->tile_on = s->tile_wanted = s->auto_form = false;  // the caller's form, not the builder's choice
+    s->tile_wanted = s->auto_form = false;  // the caller's form, not the builder's choice
+    if (s->tile_ok) {                       // its memory is the caller's again
+        CK(cudaSetDevice(s->device));
+        drop_tiles(s);
+    }
     return MGC_OK;
 }
 
 mgc_status mgc_set_tiled(mgc_sim* s, int32_t on)
 {
     if (!s) return fail(MGC_ERR_INVALID, "null handle");
-    if (on && !s->tile_ok) return fail(MGC_ERR_INVALID, "the network has no layout for the tiled step group");
-    s->tile_on = s->tile_wanted = on != 0;
-    return MGC_OK;
+    CK(cudaSetDevice(s->device));
+    s->tile_wanted = on != 0;
+    if (!on) {
+        if (s->tile_ok) drop_tiles(s);
+        return MGC_OK;
+    }
+    if (!s->tile_ok) CKS(build_tiles(s));
+    s->tile_on = s->tile_ok;
+    return s->tile_ok ? MGC_OK
+                      : fail(MGC_ERR_INVALID, "the network has no layout for the tiled step group, or no memory for it");
 }
 
 mgc_status mgc_get_step_form(mgc_sim* s, mgc_step_form* f)
@@ -205,7 +216,14 @@ mgc_status mgc_set_pull(mgc_sim* s, int32_t min_pairs)
         s->graph = nullptr;
         s->sched_graph = false;
     }
-    if (min_pairs > 0) CKS(build_in_rows(s));
+    if (min_pairs > 0) {
+        mgc_status st = build_in_rows(s);
+        if (st == MGC_ERR_NOMEM && s->tile_ok) {  // (rows asked for come before the tiles)
+            drop_tiles(s);
+            st = build_in_rows(s);
+        }
+        CKS(st);
+    }
     a.pull_min = min_pairs;
     return MGC_OK;
 }
@@ -256,6 +274,7 @@ mgc_status mgc_autotune(mgc_sim* s, int64_t steps_per_trial, mgc_tune_report* re
     if (!s->a.deferred)
         for (int g : {16, 37, 74}) cands.push_back({0, 1, g});
     const int64_t steps = (steps_per_trial + kGraphSteps - 1) / kGraphSteps * kGraphSteps;
+    if (!s->tile_ok && !sched_wanted(s)) CKS(build_tiles(s));
     s->tile_on = s->auto_form = false;
     s->persistent = 0;  // the shapes are timed as graphs of single-step kernels, step groups after
     cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -392,6 +411,7 @@ mgc_status mgc_autotune(mgc_sim* s, int64_t steps_per_trial, mgc_tune_report* re
         if (st == MGC_OK) st = mgc_sync(s);
     }
     s->tile_wanted = s->tile_on;
+    if (s->tile_ok && !s->tile_on) drop_tiles(s);
     s->persistent = rep->persistent;
     s->window = best_window;
     rep->window = s->fused ? s->window : 0;

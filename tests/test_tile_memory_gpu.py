@@ -64,3 +64,77 @@ def test_networks_are_built_without_the_tiles_memory(name):
     gc.collect()
     torch.cuda.synchronize()
     assert torch.cuda.mem_get_info()[0] > free0 - (64 << 20)
+
+
+def tiled_net():
+    args, kw = group.network(seed=7, n=4000, nx=400, k=100, delays=[15], rate=0.002)
+    return mgb.Simulator.from_arrays(*args, **dict(kw, seed=5))
+
+
+@pytest.mark.gpu
+def test_another_form_gives_the_tiles_memory_back():
+    sim = tiled_net()
+    held = sim.info()["device_bytes"]
+    copy = 2 * 4000 * 100                       # 16-bit records at least
+    sim.set_persistent(3)
+    assert sim.info()["device_bytes"] < held - copy
+    sim.set_tiled()
+    assert sim.info()["device_bytes"] == held
+    sim.set_tiled(False)
+    assert sim.info()["device_bytes"] < held - copy
+    sim.autotune(steps_per_trial=64)            # times the tiles all the same
+    assert sim.step_form()["form"] == capi.FORM_TILED and sim.info()["device_bytes"] == held
+    sim.close()
+
+
+@pytest.mark.gpu
+def test_memory_asked_for_comes_before_the_tiles():
+    """Pull steps' rows that fit without the tiles take their place."""
+    sim = tiled_net()
+    ref = tiled_net()
+    ref.set_persistent(0)
+    for s in (sim, ref):
+        s.run(100)
+        s.sync()
+    for k in range(1, 9):                       # every allocation of the rows
+        s = tiled_net()
+        mgb.fault_inject_alloc(k)
+        try:
+            s.set_pull(500)
+        finally:
+            mgb.fault_inject_alloc(0)
+        assert s.step_form()["form"] != capi.FORM_TILED
+        s.close()
+    mgb.fault_inject_alloc(1)
+    try:
+        sim.stage_raster()
+    finally:
+        mgb.fault_inject_alloc(0)
+    assert sim.step_form()["form"] != capi.FORM_TILED
+    for x, y in zip(sim.collect_raster(), ref.read_raster()):
+        assert np.array_equal(x, y)
+    for s in (sim, ref):
+        s.run(100)
+        s.sync()
+    for x, y in zip(sim.read_raster(), ref.read_raster()):
+        assert np.array_equal(x, y)
+    sim.close()
+    ref.close()
+
+
+@pytest.mark.gpu
+def test_rows_that_do_not_fit_leave_nothing_behind():
+    sim = tiled_net()
+    sim.set_persistent(3)
+    held = sim.info()["device_bytes"]
+    for k in range(1, 9):
+        mgb.fault_inject_alloc(k)
+        with pytest.raises(mgb.MgcError) as e:
+            sim.set_pull(500)
+        mgb.fault_inject_alloc(0)
+        assert e.value.status == capi.MGC_ERR_NOMEM
+        assert sim.info()["device_bytes"] == held
+    sim.set_pull(500)
+    sim.run(200)
+    sim.sync()
+    sim.close()
