@@ -408,7 +408,22 @@ mgc_status mgc_read_weights(mgc_sim* s, float* weight)
     const int64_t* src_idx = s->a.pull ? s->in_syn64 : s->csr_syn64;
     DevTmp t;
     float* out = s->weights_buf;
-    if (!out) CKS(tmp_alloc(t, &out, s->S));
+    if (!out) {
+        const mgc_status st = tmp_alloc(t, &out, s->S);
+        if (st == MGC_ERR_NOMEM) {  // a full device: a stretch at a time in host memory
+            const int64_t step = std::min<int64_t>(s->S, int64_t(1) << 22);
+            std::vector<uint2> words(step);
+            std::vector<int64_t> idx(step);
+            for (int64_t b = 0; b < s->S; b += step) {
+                const int64_t c = std::min(step, s->S - b);
+                CK(cudaMemcpy(words.data(), src_words + b, 8 * c, cudaMemcpyDeviceToHost));
+                CK(cudaMemcpy(idx.data(), src_idx + b, 8 * c, cudaMemcpyDeviceToHost));
+                for (int64_t p = 0; p < c; ++p) memcpy(&weight[idx[p]], &words[p].y, 4);
+            }
+            return MGC_OK;
+        }
+        CKS(st);
+    }
     k_weights_out<<<grid_for(s->S), 256, 0, s->stream>>>(src_words, src_idx, s->S, out);
     CK(cudaGetLastError());
     s->launches += 1;

@@ -138,3 +138,19 @@ def test_rows_that_do_not_fit_leave_nothing_behind():
     sim.run(200)
     sim.sync()
     sim.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("big", [False, True])
+def test_weights_are_read_on_a_full_device(big):
+    n, k = (20_000, 250) if big else (300, 20)       # (5e6 synapses: two stretches)
+    args, kw = group.network(seed=7, n=n, nx=40, k=k, delays=[3, 9], weights="ranged")
+    sim = mgb.Simulator.from_arrays(*args, **kw)
+    mgb.fault_inject_alloc(1)
+    try:
+        w = sim.weights()
+    finally:
+        mgb.fault_inject_alloc(0)
+    assert np.array_equal(w.view(np.int32), args[4].view(np.int32))
+    assert np.array_equal(w, sim.weights())
+    sim.close()
