@@ -479,7 +479,10 @@ mgc_status mgc_set_persistent(mgc_sim* sim, int32_t mode);
  * the same.  No reference counterpart. */
 mgc_status mgc_set_tiled(mgc_sim* sim, int32_t on);
 
-/* The form in which the next mgc_run's steps run. */
+/* The form in which the next mgc_run's steps run, if they are not few: calls of
+ * fewer than min_steps steps run in the mode of mgc_set_persistent instead of the
+ * tiled group, and calls of one or two steps in mode 2, not the windowed group in
+ * its place, since those are faster for them. */
 enum { MGC_FORM_GRAPHS = 0, MGC_FORM_BARRIER = 1, MGC_FORM_PIPELINED = 2, MGC_FORM_WINDOWED = 3,
        MGC_FORM_TILED = 4 };
 
@@ -488,6 +491,7 @@ typedef struct mgc_step_form {
     int32_t window;            /* WINDOWED, TILED: steps per window (else 0) */
     int32_t tiles;             /* TILED: blocks (else 0) */
     int32_t tile_neurons;      /* TILED: neurons of a block, in groups of four dealt to the blocks in turn */
+    int32_t min_steps;         /* TILED: the shortest call that runs in it (else 0) */
 } mgc_step_form;
 
 mgc_status mgc_get_step_form(mgc_sim* sim, mgc_step_form* form);

@@ -130,7 +130,8 @@ class Info(C.Structure):
 
 
 class StepForm(C.Structure):
-    _fields_ = [("form", C.c_int32), ("window", C.c_int32), ("tiles", C.c_int32), ("tile_neurons", C.c_int32)]
+    _fields_ = [("form", C.c_int32), ("window", C.c_int32), ("tiles", C.c_int32), ("tile_neurons", C.c_int32),
+                ("min_steps", C.c_int32)]
 
 
 _lib = None
@@ -641,7 +642,7 @@ class Simulator:
 
     def step_form(self):
         """The form in which the next steps run: form (one of FORM_*), window,
-        tiles, tile_neurons (mgc_get_step_form)."""
+        tiles, tile_neurons, min_steps (mgc_get_step_form)."""
         f = StepForm()
         check(lib().mgc_get_step_form(self._h, C.byref(f)))
         return {k: getattr(f, k) for k, _ in StepForm._fields_}

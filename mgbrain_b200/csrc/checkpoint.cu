@@ -130,6 +130,7 @@ mgc_status mgc_checkpoint_load(mgc_sim* s, const void* buf, int64_t bytes)
     }
     // a wait that ran out since left its launch's counters behind
     CKS(clear_tile_counters(s));
+    CKS(forget_tile_rings(s));  // (of another past, though perhaps of the same step)
     CK(cudaStreamSynchronize(s->stream));
     CK(cudaMemcpy(s->a.status, &zero32, 4, cudaMemcpyHostToDevice));
     if (s->a.ev_mark) {

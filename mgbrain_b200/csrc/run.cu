@@ -79,19 +79,23 @@ int graph_group_mode(const mgc_sim* s, int p) { return p == 3 ? (s->dmin >= 4 ? 
 // The builder's choice runs as the windowed group where the pipelined one
 // (minimum delay >= 4) would run: it gives the same bits and is the faster of
 // the two at every measured size and load (1.1e9 synapses quiet 4.9 against
-// 8.6 us per step, driven 49 against 57; 1e5 neurons 2.6 against 5.6).  Not
-// with fp32 sums of unequal weights of one sign (a caller's choice), whose
-// last bits follow the order of the additions, and not for partitions, whose
-// windows of minimum delay - 1 steps are a launch each.
-int group_mode(const mgc_sim* s)
+// 8.6 us per step, driven 49 against 57; 1e5 neurons 2.6 against 5.6), but for
+// calls of one or two steps (1.1e6 neurons, calls of 1, 2 and 5 steps: 21.5, 28.2
+// and 34.9 us windowed, 18.0, 27.0 and 51.7 pipelined).  Not with fp32
+// sums of unequal weights of one sign (a caller's choice), whose last bits follow
+// the order of the additions, and not for partitions, whose windows of minimum
+// delay - 1 steps are a launch each.
+int group_mode(const mgc_sim* s, int64_t steps)
 {
     const bool windowed = s->auto_form && s->persistent == 2 && !s->partition && !(s->hetero && !s->a.fx);
-    return windowed ? 3 : s->persistent;
+    return windowed && steps >= 3 ? 3 : s->persistent;
 }
 
-int32_t wanted_acc_mask(const mgc_sim* s)
+bool runs_tiled(const mgc_sim* s, int64_t steps) { return s->tile_on && steps >= s->tile_min; }
+
+int32_t wanted_acc_mask(const mgc_sim* s, int64_t steps)
 {
-    const bool wide = s->acc_buffers == kAccBuffersWide && group_mode(s) == 3 && !s->tile_on &&
+    const bool wide = s->acc_buffers == kAccBuffersWide && group_mode(s, steps) == 3 && !runs_tiled(s, steps) &&
                       s->window > kAccBuffers;
     return wide && !sched_wanted(s) ? kAccBuffersWide - 1 : kAccBuffers - 1;
 }
@@ -295,33 +299,34 @@ mgc_status mgc_run(mgc_sim* s, int64_t steps)
     }
     CK(cudaSetDevice(s->device));
     int64_t left = steps;
-    if (left > 0) CKS(set_acc_mask(s, wanted_acc_mask(s), true));
+    bool tiled = runs_tiled(s, steps);
+    if (left > 0) CKS(set_acc_mask(s, wanted_acc_mask(s, steps), true));
     if (s->a.deferred && s->fused && !s->ahead && left > 0) {
         CKS(enqueue_step(s));  // catches up the delivery, leaves ahead = true
         --left;
     }
-    if (((s->persistent && s->a.deferred) || s->tile_on) && !sched_wanted(s)) {
+    if (((s->persistent && s->a.deferred) || tiled) && !sched_wanted(s)) {
         // one cooperative launch per group: every block resident, a grid
         // barrier between steps (or the pipelined arrive/wait) instead of a launch
-        const int p = group_mode(s), v = s->fused_variant;  // (where the tiled group does not run)
+        const int p = group_mode(s, steps), v = s->fused_variant;  // (where the tiled group does not run)
         while (left > 0) {
-            int32_t n = (int32_t)std::min<int64_t>(left, s->tile_on ? kTileSteps : kPersistentSteps);
+            int32_t n = (int32_t)std::min<int64_t>(left, tiled ? kTileSteps : kPersistentSteps);
             // the schedule trace only while the scheduler's graph runs
             StepArgs ga = s->a;
             ga.trace = nullptr;
             void* args[] = {&ga, &n};
-            if (!s->tile_on)
+            if (!tiled)
                 CK(cudaMemsetAsync(s->a.bar, 0, 4 * sizeof(unsigned int), s->stream));  // clean barriers
             cudaError_t e;
-            if (s->tile_on) {
+            if (tiled) {
                 CKS(refresh_tiles(s));
                 e = launch_tiles(s, ga, n, s->tile.T);
                 if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
                     cudaGetLastError();  // not all resident here: the other step groups
-                    s->tile_wanted = false;
+                    tiled = s->tile_wanted = false;
                     drop_tiles(s);
-                    if (!s->a.deferred) break;
-                    CKS(set_acc_mask(s, wanted_acc_mask(s), true));
+                    if (!s->a.deferred || !p) break;
+                    CKS(set_acc_mask(s, wanted_acc_mask(s, steps), true));
                     continue;
                 }
             } else if (p == 3) {

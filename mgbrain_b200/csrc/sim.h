@@ -149,6 +149,7 @@ struct mgc_sim {
     bool tile_on = false;             //   whether steps run in it,
     bool tile_wanted = true;          //   whether they should: until the caller or the autotuner
                                       //   chooses another form
+    int64_t tile_min = 1;             //   the shortest call that does,
     bool tile_stale = false;          //   STDP: other forms changed the weights since its last step
     bool tile_one = false;            //   one delay, fp32 sums: 16-bit records
     size_t tile_smem = 0;             //   its dynamic shared memory
@@ -298,6 +299,8 @@ mgc_status build_tiles(mgc_sim* s);
 mgc_status refresh_tiles(mgc_sim* s);
 // One launch of the tiled group: n steps, on `blocks` blocks (its tiles).
 cudaError_t launch_tiles(mgc_sim* s, StepArgs& a, int32_t n, int32_t blocks);
+// The rings kept between launches no longer follow from the state (enqueued).
+mgc_status forget_tile_rings(mgc_sim* s);
 // The step counters and a.done as a finished launch leaves them (enqueued).
 mgc_status clear_tile_counters(mgc_sim* s);
 // In-place exclusive scan of count + 1 entries (the last becomes the total).
@@ -314,14 +317,16 @@ mgc_status build_graph(mgc_sim* s);
 mgc_status build_sched_graph(mgc_sim* s);
 bool sched_wanted(const mgc_sim* s);
 mgc_status refresh_graph(mgc_sim* s);
-// The step-group mode the next steps run in, outside the scheduler's graph and
-// the tiled group.
-int group_mode(const mgc_sim* s);
+// The step-group mode a call of `steps` steps runs in, outside the scheduler's
+// graph and the tiled group.
+int group_mode(const mgc_sim* s, int64_t steps);
+// Whether it runs in the tiled group (outside the scheduler's graph).
+bool runs_tiled(const mgc_sim* s, int64_t steps);
 // The step-group mode the scheduler's graph runs for mode p.
 int graph_group_mode(const mgc_sim* s, int p);
 // The accumulator cycle the next steps run with: 7 (eight buffers) while
 // windowed groups of more than 4 steps run, else 3.
-int32_t wanted_acc_mask(const mgc_sim* s);
+int32_t wanted_acc_mask(const mgc_sim* s, int64_t steps);
 // Switch the accumulator cycle to `mask`: with `move`, the buffer holding the
 // current step's arrivals moves to its place in the new cycle (on the
 // stream); graphs holding the old cycle are dropped.

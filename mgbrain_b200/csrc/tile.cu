@@ -15,6 +15,19 @@ constexpr int kTileRowBlock = 256;
 // the tiles are the faster form on both loads (1.1 / 3.7 against 2.6 / 4.2).
 constexpr int kTileThinNeurons = 1 << 17;
 
+// The shortest call that runs in the group.  A launch costs 15 us and more over
+// its steps (the state into shared memory and back, an exchange at the end), a step
+// of the other forms 3 to 8: calls of 1, 2, 4 and 8 steps took 20.7, 21.3, 22.5 and
+// 24.4 us in it and 14.0, 20.6, 33.0 and 58.6 pipelined (36,000 neurons, delays of 18
+// steps, 73 spikes a step).  With more neurons than threads in a tile its launch
+// costs more: 744 a tile, 34.5, 35.8, 36.6 and 37.5 against 13.2, 19.8, 30.8 and 52.7
+// (or 38 windowed).  Plastic networks (784 -> 1,600), one and two steps: 17.0 and
+// 22.4, 15.7 and 30.8 with the ring kernels.
+int64_t shortest_call(const TileArgs& t, bool stdp)
+{
+    return stdp ? 2 : 4 + (std::max(0, t.nl - kTileThreads) + 63) / 64;
+}
+
 // Records per vector.
 __host__ __device__ constexpr int vec_records(bool fx, bool one) { return !fx && one ? 4 : 2; }
 
@@ -219,12 +232,18 @@ void drop_tiles(mgc_sim* s)
 {
     cudaStreamSynchronize(s->stream);
     TileArgs& t = s->tile;
-    for (const void* p : {(const void*)t.off, t.rec, (const void*)t.we, (const void*)t.wi, (const void*)t.chain,
+    for (const void* p : {(const void*)t.off, t.rec, (const void*)t.pend, (const void*)t.pend_step, (const void*)t.we, (const void*)t.wi, (const void*)t.chain,
                           (const void*)t.list, (const void*)t.mail, (const void*)t.cnt, (const void*)t.cpos,
                           (const void*)t.in_off, (const void*)t.in_ent})
         if (p) s->release(const_cast<void*>(p));
     t = TileArgs{};
     s->tile_ok = s->tile_on = false;
+}
+
+mgc_status forget_tile_rings(mgc_sim* s)
+{
+    if (s->tile.pend_step) CK(cudaMemsetAsync(s->tile.pend_step, 0xff, sizeof(int64_t), s->stream));
+    return MGC_OK;
 }
 
 static mgc_status lay_tiles(mgc_sim* s)
@@ -256,7 +275,10 @@ static mgc_status lay_tiles(mgc_sim* s)
     // at most one vector in each segment is not full
     const size_t most = ((size_t)s->S / 2 + (size_t)s->n * T) * vec_bytes;
     const int W = stdp ? 1 : std::min(kTileWindow, s->dmin);
-    const size_t need = most + (stdp ? 12 * (size_t)s->S : 0) + ((size_t)s->n * T + 1) * 4 + kTileLists * (size_t)W * nl_of(T) * T * 4 + 32 * (size_t)T * T * kTileChunks + 16 * (size_t)a.ns;
+    const size_t ring = stdp ? 0 : (fx ? 16 : 4) * (size_t)s->dmax * tile_stride((int)nl_of(T));  // of a tile
+    const size_t need = most + (stdp ? 12 * (size_t)s->S : 0) + ((size_t)s->n * T + 1) * 4 +
+                        kTileLists * (size_t)W * nl_of(T) * T * 4 + 32 * (size_t)T * T * kTileChunks +
+                        16 * (size_t)a.ns + ring * T;
     // offsets in vectors, and in records while they are filled
     if ((int64_t)s->n * T + 1 > (int64_t)0x7fffffff || most / vec_bytes > kIndex / 2) return MGC_OK;
     size_t free_b = 0, total_b = 0;
@@ -272,6 +294,7 @@ static mgc_status lay_tiles(mgc_sim* s)
     t.dmin = s->dmin;
     t.dmax = s->dmax;
     t.ahead = s->fused ? 1 : 0;
+    s->tile_min = shortest_call(t, stdp);
     uint32_t* off;
     float *we = nullptr, *wi = nullptr, *chain = nullptr;
     CKS(s->alloc(&off, (size_t)s->n * T + 1, false));
@@ -280,6 +303,13 @@ static mgc_status lay_tiles(mgc_sim* s)
     CKS(s->alloc(&t.mail, 2 * (size_t)T * T * kTileChunks));
     t.epoch = 1;
     CKS(s->alloc(&t.cnt, 4 * kTileWindow * kTileLine));
+    if (!stdp) {
+        char* pend;
+        CKS(s->alloc(&pend, ring * T, false));
+        t.pend = pend;
+        CKS(s->alloc(&t.pend_step, 1, false));
+        CKS(forget_tile_rings(s));
+    }
     DevTmp t_deg, t_stat;
     uint32_t *indeg = nullptr, *wstat = nullptr;
     if (!fx) {

@@ -34,13 +34,19 @@
 // Input ring: the arrivals of step x in slot x % R, R = the longest delay: a
 // window's updates clear its W slots before its spikes are delivered, which
 // arrive W to W - 1 + R steps after its first step.  The group starts and
-// ends in the state of the single-step kernels: the prologue delivers the
-// spikes of the history that arrive after the first step (whose arrivals the
-// accumulators hold), the last windows' spikes are written into the
-// history, and the arrivals of the step after the last go into the
-// accumulators.  With a minimum delay of one step the single-step kernels
-// start a step without its arrivals; there the prologue includes them and
-// the accumulators stay empty.
+// ends in the state of the single-step kernels: the last windows' spikes are
+// written into the history, and the arrivals of the step after the last go into
+// the accumulators.  The later ones are kept as they stand in the ring (`pend`,
+// valid for a launch that starts at that step: `pend_step`).  A launch after
+// steps of another form delivers the history's spikes that arrive after its first
+// step (whose arrivals the accumulators hold) once more, which every call paid at
+// first: 12,000 neurons, 9.8e6 synapses of 10 to 50 steps, 2,460 spikes a step, in
+// calls of one step: 298 us a call, 45 with the kept ring.  With a minimum
+// delay of one step the single-step kernels start a step without its arrivals;
+// there the ring includes them and the accumulators stay empty.
+//
+// Events are counted by the spike's own tile, from the CSR's (source, delay)
+// offsets: those of a launch's steps, whichever launch delivered them.
 //
 // Exchange of window k: a tile sends every tile its spikes (id, step in the
 // window) in 16-byte chunks, one store each, into that tile's mailbox: {epoch of
@@ -109,6 +115,8 @@ struct TileArgs {
     uint32_t epoch;       // epoch of the launch's first window (they count on over the launches; never 0,
                           //   which the mailboxes hold at first, and never past 2^32 - 1: launch_tiles)
     int32_t* cnt;         // [4][kTileWindow] counters (tile_counter) of a window's steps' spikes; zero between launches
+    void* pend;           // [T] rings as the last launch left them (of the steps after its end),
+    int64_t* pend_step;   //   and the step they continue at (-1: none)
     // plastic networks (k_tile_stdp): rec holds single records (off counts them)
     const uint32_t* cpos;   // [S] CSR position of a record
     const uint32_t* in_off; // [T*nl + 1] plastic synapses onto each local neuron, tile after tile:
@@ -451,19 +459,18 @@ __device__ __forceinline__ void tile_update(const StepArgs& a, const TileArgs& t
 // its arrival step); j: the step's place in the batch.
 template <bool FX, bool ONE>
 __device__ __forceinline__ void tile_apply(const StepArgs& a, const TileArgs& t, const TileSmem& m, uint32_t x,
-                                           uint32_t wbits, int base, int j, int lo_rel, unsigned span, uint32_t& ev)
+                                           uint32_t wbits, int base, int j, int lo_rel, unsigned span)
 {
     if (ONE) {  // base: byte offset of the row | the sign; fillers go to the row's spare column
         if (!MGC_OK_INDEX((x >> 2) < (uint32_t)t.stride && !(x & 3u))) return;
         atomicAdd(reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(m.ring) + ((base & ~1) + x)),
                   (base & 1) ? 0x10000u : 1u);
-    } else {    // a filler's delay is past every arrival window
+    } else {    // a filler's delay is past every arrival
         const int d = (int)((x >> 16) & 0x7fffu);
         if ((unsigned)(j + d - lo_rel - 1) >= span) return;
         int row = base + d;
         if (row >= t.R) row -= t.R;
         if (!MGC_OK_INDEX(row < t.R && (x & 0xffffu) < (uint32_t)t.nl)) return;
-        ++ev;
         const int at = row * t.stride + (int)(x & 0xffffu);
         if (FX) {
             const float w = as_f(wbits);
@@ -484,19 +491,19 @@ template <> struct TileVec<true> { using type = uint4; };
 template <bool FX, bool ONE>
 __device__ __forceinline__ void tile_apply_vec(const StepArgs& a, const TileArgs& t, const TileSmem& m,
                                                const typename TileVec<FX>::type& v, int base, int j, int lo_rel,
-                                               unsigned span, uint32_t& ev)
+                                               unsigned span)
 {
     if constexpr (FX) {
-        tile_apply<FX, ONE>(a, t, m, v.x, v.y, base, j, lo_rel, span, ev);
-        tile_apply<FX, ONE>(a, t, m, v.z, v.w, base, j, lo_rel, span, ev);
+        tile_apply<FX, ONE>(a, t, m, v.x, v.y, base, j, lo_rel, span);
+        tile_apply<FX, ONE>(a, t, m, v.z, v.w, base, j, lo_rel, span);
     } else if constexpr (ONE) {
-        tile_apply<FX, ONE>(a, t, m, v.x & 0xffffu, 0u, base, j, lo_rel, span, ev);
-        tile_apply<FX, ONE>(a, t, m, v.x >> 16, 0u, base, j, lo_rel, span, ev);
-        tile_apply<FX, ONE>(a, t, m, v.y & 0xffffu, 0u, base, j, lo_rel, span, ev);
-        tile_apply<FX, ONE>(a, t, m, v.y >> 16, 0u, base, j, lo_rel, span, ev);
+        tile_apply<FX, ONE>(a, t, m, v.x & 0xffffu, 0u, base, j, lo_rel, span);
+        tile_apply<FX, ONE>(a, t, m, v.x >> 16, 0u, base, j, lo_rel, span);
+        tile_apply<FX, ONE>(a, t, m, v.y & 0xffffu, 0u, base, j, lo_rel, span);
+        tile_apply<FX, ONE>(a, t, m, v.y >> 16, 0u, base, j, lo_rel, span);
     } else {
-        tile_apply<FX, ONE>(a, t, m, v.x, 0u, base, j, lo_rel, span, ev);
-        tile_apply<FX, ONE>(a, t, m, v.y, 0u, base, j, lo_rel, span, ev);
+        tile_apply<FX, ONE>(a, t, m, v.x, 0u, base, j, lo_rel, span);
+        tile_apply<FX, ONE>(a, t, m, v.y, 0u, base, j, lo_rel, span);
     }
 }
 
@@ -596,7 +603,7 @@ struct TileSource {
 };
 
 // Delivers spikes of the steps x0, x0+1, ... to this tile's targets: the
-// records whose arrival step is in (lo, hi].  slot0: the ring slot of x0.
+// records whose arrival step is after lo.  slot0: the ring slot of x0.
 // A warp's batches run as a pipeline of three dependent loads: the spike ids
 // of the batch after next, the segment offsets of the next and the records
 // of this one are in flight together, and a lane loads kTileD vectors of each
@@ -605,20 +612,17 @@ struct TileSource {
 // a batch).  Long segments are cut for 1 << lanes_log2 lanes.
 template <bool FX, bool ONE>
 __device__ __forceinline__ void tile_deliver(const StepArgs& a, const TileArgs& t, const TileSmem& m, int64_t x0,
-                                             int slot0, int64_t lo, int64_t hi, TileSource src,
-                                             unsigned long long& events)
+                                             int slot0, int64_t lo, TileSource src)
 {
     using Vec = typename TileVec<FX>::type;
     constexpr int U = kTileU, D = FX ? kTileD / 2 : kTileD;
     const Vec* rec = reinterpret_cast<const Vec*>(t.rec);
     const int lane = threadIdx.x & 31;
     const int lg = t.lanes_log2;
-    // arrival windows relative to x0, as one unsigned comparison
-    const int64_t hr = hi - x0, lr = lo - x0;
+    // the arrivals that count, relative to x0, as one unsigned comparison
+    const int64_t lr = lo - x0;
     const int lo_rel = (int)(lr < -1 ? -1 : lr);
-    const int hi_rel = (int)(hr > 4 * kTileMaxDelay ? 4 * kTileMaxDelay : hr);
-    const unsigned span = hi_rel > lo_rel ? (unsigned)(hi_rel - lo_rel) : 0u;
-    uint32_t ev = 0;
+    const unsigned span = (unsigned)(4 * kTileMaxDelay - lo_rel);  // (a filler's delay is past it)
     // a batch of n spikes is n << lg parts of segments; `done` of them taken
     int n = 0, done = 0;
     bool more = src.begin(a, t, m, n);
@@ -707,14 +711,13 @@ __device__ __forceinline__ void tile_deliver(const StepArgs& a, const TileArgs& 
 #pragma unroll
                 for (int d = 0; d < D; ++d)
                     if (k[u] + d < e[u])
-                        tile_apply_vec<FX, ONE>(a, t, m, v[u][d], base[u], j[u], lo_rel, span, ev);
+                        tile_apply_vec<FX, ONE>(a, t, m, v[u][d], base[u], j[u], lo_rel, span);
                 k[u] += D;
                 rest |= k[u] < e[u];
             }
             if (!rest) break;
         }
     }
-    events += ev;
 }
 
 // 16 bytes as one access (neither half is seen without the other).
@@ -839,7 +842,7 @@ template <bool CUR, bool FX, bool ONE>
 __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t, int32_t nsteps)
 {
     extern __shared__ __align__(16) unsigned char tile_raw[];
-    __shared__ int abort_flag, late;  // waits that ran out: for the mailboxes, the counters
+    __shared__ int abort_flag;
     __shared__ unsigned long long blk_ev;
     __shared__ int count, npg, total;  // the tile's spikes of the window, its POISSON groups, all tiles' spikes
     __shared__ uint32_t mine[kTileInline + 2];  // (a chunk's words past the last spike are read)
@@ -854,20 +857,33 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
     int64_t rbase = rec ? *a.raster_pos : 0;
     const int64_t rstep0 = *a.raster_step0;
     const int64_t s_end = s0 + nsteps;
-    // arrivals this launch delivers and counts: (lo, hi]
+    // arrivals of this launch, whose events it counts: (lo, hi]
     const int64_t lo = t.ahead ? s0 : s0 - 1, hi = t.ahead ? s_end : s_end - 1;
     auto hs_of = [&](int64_t x) {  // history slot of a step within H of s0, or later
         int64_t h = (h0 + (x - s0)) % a.H;
         return (int32_t)(h < 0 ? h + a.H : h);
     };
     unsigned long long ev = 0;
+    auto events_of = [&](int32_t id, int64_t x) {  // a spike's synapses whose arrival is in (lo, hi]
+        if (ONE) return (unsigned long long)(x + t.dmin > lo && x + t.dmin <= hi ? a.row_ptr[id + 1] - a.row_ptr[id] : 0);
+        const int64_t a0 = lo - x - t.dmin + 1, a1 = hi - x - t.dmin + 1;
+        const int64_t* bk = a.bucket + (size_t)id * a.D;
+        const int k0 = (int)(a0 < 0 ? 0 : a0 > a.D ? a.D : a0), k1 = (int)(a1 < 0 ? 0 : a1 > a.D ? a.D : a1);
+        return (unsigned long long)(k0 < k1 ? bk[k1] - bk[k0] : 0);
+    };
+    // the ring, words of 16 bytes (a row's entries are a multiple of 4)
+    const int ring_words = (FX ? 4 : 1) * t.R * t.stride / 4;
+    uint4* pend = reinterpret_cast<uint4*>(t.pend) + (size_t)tile * ring_words;
+    const bool kept = *t.pend_step == s0;
 
-    // state of the tile, empty ring
+    // state of the tile, its ring
     {
-        uint32_t* z = reinterpret_cast<uint32_t*>(m.ring);
-        const int words = (FX ? 4 : 1) * t.R * t.stride;
-#pragma unroll 1
-        for (int k = tid; k < words; k += blockDim.x) z[k] = 0;
+        uint4* z = reinterpret_cast<uint4*>(m.ring);
+#pragma unroll 4
+        for (int k = tid; k < ring_words; k += blockDim.x) {
+            const uint4 v = __ldcg(pend + k);  // (loaded before it is known whether it counts)
+            z[k] = kept ? v : make_uint4(0, 0, 0, 0);
+        }
 #pragma unroll 1
         for (int i = tid; i < t.nl; i += blockDim.x) {
             const int32_t gi = tile_neuron(t, i, tile);
@@ -891,7 +907,6 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
         if (tid < 4 * kTileWindow) ctot[tid / kTileWindow][tid % kTileWindow] = 0;
         if (tid == 0) {
             abort_flag = tile_refused(a);
-            late = 0;
             blk_ev = 0;
             count = npg = total = 0;
         }
@@ -905,27 +920,34 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
     }
     __syncthreads();
     const int n_pg = npg;
-    // prologue: the spikes of the last R steps before s0 that arrive later
+    // the last R steps before s0: their spikes that arrive later, when the ring was
+    // not kept, and the events of this launch's steps, a warp a step or part of one
     {
         const int64_t x0 = s0 - t.R > 0 ? s0 - t.R : 0;
         const int nst = (int)(s0 - x0);
+        if (!kept) {
 #pragma unroll 1
-        for (int j = tid; j < nst; j += blockDim.x) m.cnt[j] = __ldcg(a.hist_cnt + hs_of(x0 + j));
-        __syncthreads();
-        TileSource src;
-        src.listed(TileSource::kHistory, nst, hs_of(x0));
-        tile_deliver<FX, ONE>(a, t, m, x0, (int)(x0 % t.R), lo, hi, src, ev);
-        if (ONE)  // whole rows, counted by one block a step
-            for (int j = tile; j < nst; j += t.T) {
-                const int64_t x = x0 + j;
-                if (x + t.dmin <= lo || x + t.dmin > hi) continue;
+            for (int j = tid; j < nst; j += blockDim.x) m.cnt[j] = __ldcg(a.hist_cnt + hs_of(x0 + j));
+            __syncthreads();
+            TileSource src;
+            src.listed(TileSource::kHistory, nst, hs_of(x0));
+            tile_deliver<FX, ONE>(a, t, m, x0, (int)(x0 % t.R), lo, src);
+        }
+        const int lane = tid & 31, warps = t.T * (int)(blockDim.x >> 5);
+        const int each = nst > 0 && warps > nst ? warps / nst : 1;  // warps of a step
+        const int h_first = hs_of(x0);
 #pragma unroll 1
-                for (int q = tid; q < m.cnt[j]; q += blockDim.x) {
-                    const int32_t id = __ldcg(a.hist_ids + (size_t)hs_of(x) * (size_t)a.n_src + q);
-                    if (MGC_OK_INDEX(id >= 0 && id < a.n_src))
-                        ev += (unsigned long long)(a.row_ptr[id + 1] - a.row_ptr[id]);
-                }
+        for (int w = tile + (tid >> 5) * t.T; w < nst * each; w += warps) {
+            const int j = w / each, part = w - j * each;
+            if (x0 + j + t.dmin > hi || x0 + j + t.dmax <= lo) continue;
+            const int h = h_first + j, hs = h >= a.H ? h - a.H : h;
+            const int c = __ldcg(a.hist_cnt + hs);
+#pragma unroll 1
+            for (int q = part * 32 + lane; q < c; q += each * 32) {
+                const int32_t id = __ldcg(a.hist_ids + (size_t)hs * (size_t)a.n_src + q);
+                if (MGC_OK_INDEX(id >= 0 && id < a.n_src)) ev += events_of(id, x0 + j);
             }
+        }
         __syncthreads();
     }
     // the spikes of window k (w steps from x0): their raster places, and the
@@ -947,7 +969,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
             const int64_t x = x0 + j, rb = rbase + stot[j] + at;
             if (rec && rb < a.raster_ids_cap) a.raster_ids[rb] = id;
             if (x > s_end - a.H && MGC_OK_INDEX(at < a.n_src)) a.hist_ids[(size_t)hs_last(x) * (size_t)a.n_src + at] = id;
-            if (ONE && x + t.dmin <= hi) ev += (unsigned long long)(a.row_ptr[id + 1] - a.row_ptr[id]);
+            ev += events_of(id, x);
         }
         if (tile == 0 && tid < w) {
             const int64_t x = x0 + tid;
@@ -963,24 +985,26 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
         }
         rbase += stot[w];
     };
-    // running sums of window k's step totals (n_all in all), by the first warp;
-    // now: the counters as read before
+    // running sums of window k's step totals (n_all in all), by the last warp, which
+    // has the fewest spikes to deliver; now: the counters as read before
+    const int last = tid - (kTileThreads - 32);
+    int gave_up = 0;  // (counters that never added up)
     auto totals = [&](int k, int w, int n_all, int32_t now) {
-        if (tid < 32) {
+        if (last >= 0) {
             int c;
             for (unsigned it = 0;;) {
-                c = tid < w ? now - ctot[k & 3][tid] : 0;
+                c = last < w ? now - ctot[k & 3][last] : 0;
 #pragma unroll
                 for (int o = 1; o < kTileWindow; o <<= 1) {
                     const int v = __shfl_up_sync(0xffffffffu, c, o);
-                    if (tid >= o) c += v;
+                    if (last >= o) c += v;
                 }
-                if (__shfl_sync(0xffffffffu, c, kTileWindow - 1) == n_all || !tile_again(a, it, &late)) break;
-                if (tid < w) now = tile_count(t, k, tid);
+                if (__shfl_sync(0xffffffffu, c, kTileWindow - 1) == n_all || !tile_again(a, it, &gave_up)) break;
+                if (last < w) now = tile_count(t, k, last);
             }
-            if (tid < w) ctot[k & 3][tid] = now;
-            if (tid < w) stot[tid + 1] = c;
-            if (tid == 0) stot[0] = 0;
+            if (last < w) ctot[k & 3][last] = now;
+            if (last < w) stot[last + 1] = c;
+            if (last == 0) stot[0] = 0;
         }
     };
     int slot = (int)(s0 % t.R);
@@ -997,7 +1021,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
         int place = 0;
         if (tid >= 32 && tid < 32 + wl && scnt[tid - 32])
             place = atomicAdd(tile_counter(t, k, tid - 32), scnt[tid - 32]);
-        const int32_t early = k > 0 && tid < w_prev ? tile_count(t, k - 1, tid) : 0;
+        const int32_t early = k > 0 && last >= 0 && last < w_prev ? tile_count(t, k - 1, last) : 0;
         const uint32_t* lists = t.list + (size_t)(k % kTileLists) * t.T * list_len;
         if (!tile_gather(a, t, m, k, lists, list_len, &total, &abort_flag)) return;
         if (tid >= 32 && tid < 32 + kTileWindow) {
@@ -1012,9 +1036,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
             src.gathered(n_prev);
         else
             src.listed(TileSource::kTiles, t.T, k);
-        tile_deliver<FX, ONE>(a, t, m, w0, slot, lo, hi, src, ev);
-        __syncthreads();
-        if (late) return;
+        tile_deliver<FX, ONE>(a, t, m, w0, slot, lo, src);
+        if (__syncthreads_or(gave_up)) return;
         if (tid == 0) total = 0;
         if (k > 0) record(k - 1, w0 - w_prev, w_prev, c_prev);
         c_prev = c_now;
@@ -1026,16 +1049,16 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
     // the last window's raster and history: an empty window makes its counters final
     tile_publish(t, k, 0, mine);
     if (!tile_gather(a, t, m, k, t.list, 0, &total, &abort_flag)) return;
-    totals(k - 1, w_prev, n_prev, tid < w_prev ? tile_count(t, k - 1, tid) : 0);
-    __syncthreads();
-    if (late) return;
+    totals(k - 1, w_prev, n_prev, last >= 0 && last < w_prev ? tile_count(t, k - 1, last) : 0);
+    if (__syncthreads_or(gave_up)) return;
     record(k - 1, w0 - w_prev, w_prev, c_prev);
     // back to the single-step form: the state, and the arrivals of s_end
 #pragma unroll 1
     for (int i = tid; i < t.nl; i += blockDim.x) {
         const int32_t gi = tile_neuron(t, i, tile);
         if (gi >= a.ns) continue;
-        if (m.type[i] == kPOISSON) continue;  // keeps its probability, ignores its input
+        if (m.type[i] == kPOISSON || m.type[i] == kRAW) continue;  // they keep V and ignore their input (whose
+                                                                   // ring words may run over: 32 bits each)
         a.V[gi] = m.V[i];
         a.refrac[gi] = m.rf[i];
         if (CUR) {
@@ -1045,17 +1068,23 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
         if (t.ahead) {
             const size_t at = (size_t)slot * t.stride + i;
             if (FX) {
-                const unsigned long long* e = reinterpret_cast<const unsigned long long*>(m.ring);
+                unsigned long long* e = reinterpret_cast<unsigned long long*>(m.ring);
                 acc_buf<FX>(a, a.acc_e, s_end)[gi] = (typename AccT<FX>::type)e[at];
                 acc_buf<FX>(a, a.acc_i, s_end)[gi] = (typename AccT<FX>::type)e[(size_t)t.R * t.stride + at];
+                e[at] = e[(size_t)t.R * t.stride + at] = 0;
             } else {
-                const uint32_t c = reinterpret_cast<const uint32_t*>(m.ring)[at];
+                uint32_t* ring = reinterpret_cast<uint32_t*>(m.ring);
+                const uint32_t c = ring[at];
                 acc_buf<FX>(a, a.acc_e, s_end)[gi] = (typename AccT<FX>::type)chain_sum(c & 0xffffu, m.we[i], m.tab);
                 acc_buf<FX>(a, a.acc_i, s_end)[gi] =
                     (typename AccT<FX>::type)chain_sum(c >> 16, m.wi[i], m.tab ? m.tab + kTileTable : nullptr);
+                ring[at] = 0;
             }
         }
     }
+    __syncthreads();
+#pragma unroll 4
+    for (int k = tid; k < ring_words; k += blockDim.x) pend[k] = reinterpret_cast<const uint4*>(m.ring)[k];
     if (ev) atomicAdd(&blk_ev, ev);
     __syncthreads();
     if (tid == 0 && blk_ev) atomicAdd(a.events, blk_ev);
@@ -1069,6 +1098,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
         a.slots[0] = (int32_t)((slot0 + nsteps) % a.M);
         a.slots[1] = h_end;
         *a.step = s_end;
+        *t.pend_step = s_end;
     }
 }
 
@@ -1225,16 +1255,14 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile_stdp(StepArgs a, TileA
         tile_publish(t, k, c_now, mine);
         int place = 0;
         if (tid == 32 && c_now) place = atomicAdd(tile_counter(t, k, 0), c_now);
-        const int32_t early = k > 0 && tid == 0 ? tile_count(t, k - 1, 0) : 0;
+        const int32_t early = k > 0 && tid == kTileThreads - 1 ? tile_count(t, k - 1, 0) : 0;
         if (!tile_gather(a, t, m, k, tile_list(t, k, 0), list_len, &total, &abort_flag)) return;
         if (tid == 32) {
             sbase[k & 1] = place - ctot[k & 3];
             scnt[0] = 0;
         }
-        if (tid == 0) {
-            count = 0;
-            if (k > 0) total_of(k - 1, n_prev, early);
-        }
+        if (tid == 0) count = 0;
+        if (k > 0 && tid == kTileThreads - 1) total_of(k - 1, n_prev, early);  // (it has the fewest spikes to deliver)
         n_prev = total;
         each_spike(k, tid, blockDim.x, [&](int32_t id) {
             if (!MGC_OK_INDEX(id >= 0 && id < a.n)) return;

@@ -187,12 +187,12 @@ mgc_status mgc_set_tiled(mgc_sim* s, int32_t on)
 mgc_status mgc_get_step_form(mgc_sim* s, mgc_step_form* f)
 {
     if (!s || !f) return fail(MGC_ERR_INVALID, "null argument");
-    *f = mgc_step_form{MGC_FORM_GRAPHS, 0, 0, 0};
+    *f = mgc_step_form{};  // MGC_FORM_GRAPHS
     if (sched_wanted(s)) return MGC_OK;
     if (s->tile_on) {
-        *f = mgc_step_form{MGC_FORM_TILED, s->tile.W, s->tile.T, s->tile.nl};
+        *f = mgc_step_form{MGC_FORM_TILED, s->tile.W, s->tile.T, s->tile.nl, (int32_t)s->tile_min};
     } else if (s->a.deferred) {
-        f->form = group_mode(s);
+        f->form = group_mode(s, kPersistentSteps);
         f->window = f->form == MGC_FORM_WINDOWED ? s->window : 0;
     }
     return MGC_OK;

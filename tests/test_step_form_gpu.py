@@ -67,7 +67,7 @@ def test_forms_chosen_and_taken_back():
     ref.close()
     sim = make(spec)                      # never told a mode: the windowed group in the place of 2
     sim.set_tiled(False)
-    assert sim.info()["persistent"] == 2 and sim.step_form() == dict(form=3, window=8, tiles=0, tile_neurons=0)
+    assert sim.info()["persistent"] == 2 and sim.step_form() == dict(form=3, window=8, tiles=0, tile_neurons=0, min_steps=0)
     sim.close()
 
 
