@@ -534,8 +534,8 @@ mgc_status finish_build(mgc_sim* s)
         s->fused_variant = 1;
         // step groups by default (faster than one launch per step on every
         // measured load); the pipelined form needs a minimum delay >= 4.
-        // The windowed form is faster on the measured loads; the autotuner
-        // or the caller selects it
+        // Until the caller or the autotuner chooses a mode, the tiled group
+        // (build_tiles) or the windowed one (group_mode) runs in its place
         s->persistent = s->fused ? (s->dmin >= 4 ? 2 : 1) : 1;
         if (!s->fused) CKS(s->alloc(&a.bar, 4));  // the grid barrier's arrivals and generation
         if (s->fused) {

@@ -267,6 +267,12 @@ static mgc_status lay_tiles(mgc_sim* s)
         if (stdp) return nl < 0x10000 && tile_stdp_bytes((int)nl, s->dmax, T, cur, s->n) <= room;
         return nl < (one ? 0x3fff : 0x10000) && tile_smem_bytes((int)nl, s->dmax, T, fx, cur, !fx) <= room;
     };
+    // As many tiles as SMs, fewer only where a mean segment would hold less than half
+    // a record: the more tiles, the fewer events a tile (us a step on 16, 32, 64, 100
+    // and 148 tiles: volleys of 11,000 neurons 3.41, 2.83, 1.99, 1.59, 1.36; 24 networks
+    // in one batch 2.92, 2.93, 0.96, 0.76, 0.62).  Windows of one step are mostly
+    // exchange, whose cost grows with the tiles: 4,000 neurons 3.38, 3.09, 2.96, 3.02,
+    // 3.18, so up to 7 % are left there.
     int T = (int)std::max<int64_t>(1, std::min<int64_t>({(int64_t)sms, groups, 2 * s->S / s->n}));
     while (T < sms && !fits(T)) ++T;
     const int64_t avg = s->S / ((int64_t)s->n * T);  // records per segment

@@ -79,9 +79,9 @@
 //
 // Measured per step, the faster of the other step groups and this one: 4,000
 // neurons, minimum delay 1: 6.5 and 3.2 us; 11,000 neurons, windows of 15 steps
-// quiet: 5.0 and 0.31, with volleys: 8.7 and 1.35; balanced networks of 1e8
+// quiet: 5.0 and 0.31, with volleys: 8.7 and 1.36; balanced networks of 1e8
 // synapses, quiet: 6.6 and 0.98, and of 3e7 at POISSON rates of 1 kHz: 20.9 and
-// 4.7; 9,000 neurons with a range of delays: 7.8 and 1.1.
+// 4.6; 9,000 neurons with a range of delays: 7.8 and 1.1.
 #pragma once
 #include <type_traits>
 
@@ -1119,7 +1119,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) k_tile(StepArgs a, TileArgs t
 // Bound by the step's chain of dependent accesses: exchange, segment
 // offsets, records, and after a spike of its own the incoming list and its
 // weights.  784 -> 1,600 plastic network, 1.9e4 events a step: 12.1 us a step
-// with the single-step ring kernels, 5.2 here.
+// with the single-step ring kernels, 5.1 here.
 // ---------------------------------------------------------------------------
 struct TileStdpSmem {
     int32_t* lf;       // [n] last spike of every neuron
