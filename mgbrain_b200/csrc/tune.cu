@@ -392,6 +392,8 @@ mgc_status mgc_autotune(mgc_sim* s, int64_t steps_per_trial, mgc_tune_report* re
     // the tiled step group, where the network has its layout: the report keeps
     // the fastest of the other forms, which runs when the tiles are turned off
     if (s->tile_ok && st == MGC_OK && !sched_wanted(s)) {
+        const int64_t shortest = s->tile_min;
+        s->tile_min = 1;  // (the trial's runs are in the group, however short)
         s->tile_on = true;
         st = mgc_run(s, kGraphSteps);
         if (st == MGC_OK) {
@@ -408,6 +410,7 @@ mgc_status mgc_autotune(mgc_sim* s, int64_t steps_per_trial, mgc_tune_report* re
             else
                 s->tile_on = false;
         }
+        s->tile_min = shortest;
         if (st == MGC_OK) st = mgc_sync(s);
     }
     s->tile_wanted = s->tile_on;
