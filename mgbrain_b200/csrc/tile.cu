@@ -15,6 +15,17 @@ constexpr int kTileRowBlock = 256;
 // the tiles are the faster form on both loads (1.1 / 3.7 against 2.6 / 4.2).
 constexpr int kTileThinNeurons = 1 << 17;
 
+// Networks with several delays whose segment offsets (4 bytes per neuron and tile)
+// take more than this keep the other step groups: the look-ups, one per spike and
+// tile, then miss L2 (126 MB).  Inputs at 20, 100, 200 and 500 Hz, in-degree 1,000,
+// delays of 4 to 8 steps, us a step here and (in brackets) in the other groups:
+// 220,000 neurons (130 MB) 2.1, 4.0, 11.1 and 26.8 (5.6, 7.8, 13.3, 25.6), 275,000
+// (163 MB) 2.3, 4.9, 14.4 and 33.1 (5.8, 9.6, 14.6, 29.6), 330,000 (195 MB) 2.5, 5.9,
+// 17.8 and 39.9 (5.9, 10.5, 15.9, 34.1), 550,000 3.4, 11.2, 31.3 and 77.3 (7.9, 12.3,
+// 22.4, 65.1).  With one delay the group stays the faster one at 200 Hz (550,000
+// neurons, delay 3: 21.6 against 23.7): a quarter of the record bytes.
+constexpr int64_t kTileOffsetBytes = 160 << 20;
+
 // The shortest call that runs in the group.  A launch costs 15 us and more over
 // its steps (the state into shared memory and back, an exchange at the end), a step
 // of the other forms 3 to 8: calls of 1, 2, 4 and 8 steps took 20.7, 21.3, 22.5 and
@@ -277,6 +288,8 @@ static mgc_status lay_tiles(mgc_sim* s)
     while (T < sms && !fits(T)) ++T;
     const int64_t avg = s->S / ((int64_t)s->n * T);  // records per segment
     if (!fits(T) || 2 * s->S / T < s->n || (avg < 4 && s->n > kTileThinNeurons)) return MGC_OK;
+    auto offsets_fit = [&] { return one || 4 * (int64_t)s->n * T <= kTileOffsetBytes; };
+    if (!offsets_fit()) return MGC_OK;
     const size_t vec_bytes = fx ? 16 : 8;
     // at most one vector in each segment is not full
     const size_t most = ((size_t)s->S / 2 + (size_t)s->n * T) * vec_bytes;
@@ -349,6 +362,10 @@ static mgc_status lay_tiles(mgc_sim* s)
     CKS(count());
     if (one && h[5]) {  // a source with synapses of both signs: a sign in every record
         one = false;
+        if (!offsets_fit()) {
+            drop_tiles(s);
+            return MGC_OK;
+        }
         CK(cudaMemsetAsync(indeg, 0, 4 * (size_t)a.ns, s->stream));
         CKS(count());
     }

@@ -132,3 +132,21 @@ def test_mailbox_edges_over_windows_of_four_steps(groups):
     sim.close()
     ref = group.run(spec, [100, 57], [0, None], {})
     group.same(ref, group.run(spec, [100, 57], [None, None], {}))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,delays,form", [(200_000, (5, 8), capi.FORM_TILED), (300_000, (5, 8), capi.FORM_WINDOWED),
+                                           (300_000, (8, 8), capi.FORM_TILED)])
+def test_offsets_beyond_l2_keep_the_other_groups(n, delays, form):
+    """Large networks with several delays: the tiles' offsets would miss L2."""
+    lif = group.LIFC
+    pops = [(0, n, mgb.LIFB), (n, n // 10, mgb.POISSON)]
+    projs = [(0, 0, 600, 1e-4, *delays), (1, 0, 60, 1e-4, *delays)]
+    rate = np.zeros(n + n // 10, np.float32)
+    rate[n:] = 0.01
+    sim = mgb.Simulator.fixed_indegree(pops, projs, lif, rate=rate, seed=3, conn_seed=2)
+    assert sim.step_form()["form"] == form
+    sim.run(30)
+    sim.sync()
+    assert sim.step_form()["form"] == form
+    sim.close()
