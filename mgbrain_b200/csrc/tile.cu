@@ -23,8 +23,27 @@ constexpr int kTileThinNeurons = 1 << 17;
 // (163 MB) 2.3, 4.9, 14.4 and 33.1 (5.8, 9.6, 14.6, 29.6), 330,000 (195 MB) 2.5, 5.9,
 // 17.8 and 39.9 (5.9, 10.5, 15.9, 34.1), 550,000 3.4, 11.2, 31.3 and 77.3 (7.9, 12.3,
 // 22.4, 65.1).  With one delay the group stays the faster one at 200 Hz (550,000
-// neurons, delay 3: 21.6 against 23.7): a quarter of the record bytes.
+// neurons, delay 3: 21.6 against 23.7): a quarter of the record bytes.  So it does with
+// a minimum delay of one step, where the others pay two barriers a step (330,000
+// neurons, delays of 1 to 5 steps: 7.1, 10.0, 20.5 and 50.5 against 9.6, 14.0, 25.2 and
+// 57.2; 495,000 at 200 Hz 30.8 against 26.9, below that 1.2 to 1.3 times as fast).
 constexpr int64_t kTileOffsetBytes = 160 << 20;
+
+// The same for networks with fixed-point sums, whose records take 8 bytes: above this
+// many synapses the records a driven step reads (with the vectors' padding more than
+// the CSR's) outweigh the exchanges saved.  In-degree 1,000, inputs at 20, 100, 200 and
+// 500 Hz, delays of 5 to 8 steps: 4.4e7 synapses 1.4, 4.3, 7.7 and 17.9 us a step (7.5,
+// 8.6, 9.2, 14.0), 5.5e7 1.4, 5.2, 9.4 and 24.9 (7.6, 8.1, 9.5, 16.2), 6.6e7 1.5, 5.9,
+// 11.2 and 28.4 (7.5, 8.8, 10.1, 18.2); delays of 10 to 30, 5.5e7 at 200 Hz 11.3 (9.7).
+// Not with a minimum delay of one step (1.4e8 synapses at 200 Hz 29 against 52 to 67).
+constexpr int64_t kTileFixedSynapses = 48 << 20;
+
+// Plastic networks: a tile takes its own spikes' incoming plastic synapses one spike
+// after another, so long lists keep the ring kernels.  us a step here and (there), the
+// inputs at 32 Hz in the mean: 2,000 plastic inputs onto each of 3,000 neurons 7.9 (11.9),
+// 3,000 onto 3,000 9.7 (12.7), 4,000 onto 4,000 23.3 (19.6); at 127 Hz 15.4 (14.5), 27.7
+// (20.9), 33.8 (24.2).
+constexpr uint32_t kTilePlasticInputs = 3072;
 
 // The shortest call that runs in the group.  A launch costs 15 us and more over
 // its steps (the state into shared memory and back, an exchange at the end), a step
@@ -288,8 +307,8 @@ static mgc_status lay_tiles(mgc_sim* s)
     while (T < sms && !fits(T)) ++T;
     const int64_t avg = s->S / ((int64_t)s->n * T);  // records per segment
     if (!fits(T) || 2 * s->S / T < s->n || (avg < 4 && s->n > kTileThinNeurons)) return MGC_OK;
-    auto offsets_fit = [&] { return one || 4 * (int64_t)s->n * T <= kTileOffsetBytes; };
-    if (!offsets_fit()) return MGC_OK;
+    auto offsets_fit = [&] { return !s->fused || one || 4 * (int64_t)s->n * T <= kTileOffsetBytes; };
+    if (!offsets_fit() || (fx && s->fused && s->S > kTileFixedSynapses)) return MGC_OK;
     const size_t vec_bytes = fx ? 16 : 8;
     // at most one vector in each segment is not full
     const size_t most = ((size_t)s->S / 2 + (size_t)s->n * T) * vec_bytes;
@@ -396,8 +415,19 @@ static mgc_status lay_tiles(mgc_sim* s)
         CKS(tmp_alloc(t_at, &at, locals + 1));
         k_tile_fill_stdp<<<grid, kTileRowBlock, 0, s->stream>>>(a.row_ptr, a.syn, a.plastic, s->n, T, t.nl, a.tmask,
                                                                 a.tbits, off, srec, cpos, in_off);
+        uint32_t n_in = 0, longest = 0;
+        DevTmp t_max;
+        uint32_t* d_max;
+        CKS(tmp_alloc(t_max, &d_max, 1));
+        CK(cudaMemsetAsync(d_max, 0, 4, s->stream));
+        k_max_u32<<<grid_for(locals), 256, 0, s->stream>>>(in_off, locals, d_max);
+        CK(cudaMemcpyAsync(&longest, d_max, 4, cudaMemcpyDeviceToHost, s->stream));
+        CK(cudaStreamSynchronize(s->stream));
+        if (longest > kTilePlasticInputs) {
+            drop_tiles(s);
+            return MGC_OK;
+        }
         CKS(scan_offsets(in_off, locals, s->stream));
-        uint32_t n_in = 0;
         CK(cudaMemcpyAsync(&n_in, in_off + locals, 4, cudaMemcpyDeviceToHost, s->stream));
         CK(cudaMemcpyAsync(at, in_off, 4 * (size_t)locals, cudaMemcpyDeviceToDevice, s->stream));
         CK(cudaStreamSynchronize(s->stream));

@@ -136,7 +136,7 @@ def test_mailbox_edges_over_windows_of_four_steps(groups):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("n,delays,form", [(200_000, (5, 8), capi.FORM_TILED), (300_000, (5, 8), capi.FORM_WINDOWED),
-                                           (300_000, (8, 8), capi.FORM_TILED)])
+                                           (300_000, (8, 8), capi.FORM_TILED), (300_000, (1, 4), capi.FORM_TILED)])
 def test_offsets_beyond_l2_keep_the_other_groups(n, delays, form):
     """Large networks with several delays: the tiles' offsets would miss L2."""
     lif = group.LIFC
@@ -150,3 +150,43 @@ def test_offsets_beyond_l2_keep_the_other_groups(n, delays, form):
     sim.sync()
     assert sim.step_form()["form"] == form
     sim.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,dmin,form", [(45_000, 5, capi.FORM_TILED), (60_000, 5, capi.FORM_WINDOWED),
+                                         (60_000, 1, capi.FORM_TILED)])
+def test_large_fixed_point_networks_keep_the_other_groups(n, dmin, form):
+    pops = [(0, n, mgb.LIFB), (n, n // 10, mgb.POISSON)]
+    projs = [(0, 0, 800, 1e-4, dmin, 8), (1, 0, 100, 3e-4, dmin, 8)]     # unequal weights of one sign
+    rate = np.zeros(n + n // 10, np.float32)
+    rate[n:] = 0.01
+    sim = mgb.Simulator.fixed_indegree(pops, projs, group.LIFC, rate=rate, seed=3, conn_seed=2)
+    assert sim.info()["accumulation"] == mgb.ACC_FIXED and sim.step_form()["form"] == form
+    sim.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("inputs,form", [(3000, capi.FORM_TILED), (3200, capi.FORM_GRAPHS)])
+def test_long_plastic_lists_keep_the_ring_kernels(inputs, form):
+    n = 64
+    types = np.full(inputs + n, mgb.LIFB, np.int8)
+    types[:inputs] = mgb.POISSON
+    src = np.tile(np.arange(inputs, dtype=np.int32), n)
+    tar = np.repeat(np.arange(inputs, inputs + n, dtype=np.int32), inputs)
+    rate = np.where(types == mgb.POISSON, 0.05, 0.0).astype(np.float32)
+    lif = np.zeros(30, np.float32)
+    lif[0], lif[4], lif[8], lif[9] = 5e-4, 20.0, 0.002, 0.02
+    outs = []
+    for choice in (0, None):
+        sim = mgb.Simulator.from_arrays(inputs + n, types, src, tar, np.full(len(src), 0.2, np.float32),
+                                        np.ones(len(src), np.int32), lif, plastic.STDP, rate=rate, stdp=True, seed=3)
+        assert sim.step_form()["form"] == form
+        if choice is not None:
+            sim.set_persistent(choice)
+        sim.run(60)
+        sim.sync()
+        outs.append((sim.read_raster(), sim.weights()))
+        sim.close()
+    for x, y in zip(outs[0][0], outs[1][0]):
+        assert np.array_equal(x, y)
+    assert np.array_equal(outs[0][1].view(np.int32), outs[1][1].view(np.int32))
