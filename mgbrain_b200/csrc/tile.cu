@@ -32,11 +32,12 @@ constexpr int64_t kTileOffsetBytes = 160 << 20;
 // The same for networks with fixed-point sums, whose records take 8 bytes: above this
 // many synapses the records a driven step reads (with the vectors' padding more than
 // the CSR's) outweigh the exchanges saved.  In-degree 1,000, inputs at 20, 100, 200 and
-// 500 Hz, delays of 5 to 8 steps: 4.4e7 synapses 1.4, 4.3, 7.7 and 17.9 us a step (7.5,
-// 8.6, 9.2, 14.0), 5.5e7 1.4, 5.2, 9.4 and 24.9 (7.6, 8.1, 9.5, 16.2), 6.6e7 1.5, 5.9,
-// 11.2 and 28.4 (7.5, 8.8, 10.1, 18.2); delays of 10 to 30, 5.5e7 at 200 Hz 11.3 (9.7).
-// Not with a minimum delay of one step (1.4e8 synapses at 200 Hz 29 against 52 to 67).
-constexpr int64_t kTileFixedSynapses = 48 << 20;
+// 500 Hz, delays of 5 to 8 steps: 4e7 synapses 1.4, 4.3, 7.7 and 17.9 us a step (7.5,
+// 8.6, 9.2, 14.0), 5e7 1.4, 5.2, 9.4 and 24.9 (7.6, 8.1, 9.5, 16.2), 6e7 1.5, 5.9, 11.2
+// and 28.4 (7.5, 8.8, 10.1, 18.2); delays of 10 to 30 at 200 Hz, 4e7 7.3 (9.0), 4.5e7
+// 10.3 (9.3).  Not with a minimum delay of one step (1.25e8 synapses at 200 Hz 29
+// against 52 to 67).
+constexpr int64_t kTileFixedSynapses = 40 << 20;
 
 // Plastic networks: a tile takes its own spikes' incoming plastic synapses one spike
 // after another, so long lists keep the ring kernels.  us a step here and (there), the
